@@ -4,18 +4,18 @@
 // follows src/gpu_search_v42.cu:354-391, :525-594), made by sm_103a kernels
 // instead of host threads, so that opening a handle needs no host pass over
 // 10^7 integers and no upload of the 3.4 GB cache:
-//   1. spf[x]: trial division of every x by the primes up to sqrt(N) (those
-//      few hundred primes come from a host sieve), one thread per x;
+//   1. spf[x]: a sieve in shared-memory tiles over the primes up to sqrt(N)
+//      (those few hundred primes come from a host sieve);
 //   2. prime-power table: per split prime p its block size (sum over a of
-//      4a+1, a <= 2 log_p N), an exclusive scan for pp_base, then a warp per
-//      p finds pi = u + iv (smallest u, as the host) and writes
+//      4a+1, a <= 2 log_p N), an exclusive scan for pp_base, then a thread per
+//      p finds pi = u + iv (smallest u, as the host) and a warp per p writes
 //      pi^r conj(pi)^(4a-r) for every a and r, exact and hot;
 //   3. segment sizes (W(x)-1)/2 + 1 from the factorisation of x, an exclusive
 //      scan for seg_off;
-//   4. one thread per x writes its free set and central value, enumerating the
-//      free vectors in the host's order with an odometer over the digits of
-//      the later primes (64-bit products: every partial product divides x^2 in
-//      the Gaussian integers, so its coordinates are at most x^2 < 2^50).
+//   4. one thread per record decodes its free vector (or the central value)
+//      from its place in x's segment, in the host's order (64-bit products:
+//      every partial product divides x^2 in the Gaussian integers, so its
+//      coordinates are at most x^2 < 2^50).
 // The host keeps copies of spf and seg_off (the item builder reads them).
 #include <cuda_runtime.h>
 #include <math.h>
@@ -79,22 +79,44 @@ __device__ Factors factor(const uint32_t* spf, uint32_t x) {
     return f;
 }
 
-__global__ void sieve_kernel(uint32_t* spf, uint32_t n, const uint32_t* primes, uint32_t nprimes) {
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x <= n; x += gridDim.x * blockDim.x) {
-        if (x < 2) {
-            spf[x] = x;  // spf[0] = 0, spf[1] = 1
-            continue;
-        }
-        uint32_t s = x;
-        for (uint32_t i = 0; i < nprimes; ++i) {
-            const uint32_t p = primes[i];
-            if (p * p > x) break;
-            if (x % p == 0) {
-                s = p;
-                break;
+// Smallest prime factors, kSieveTile integers per CTA in shared memory: the
+// primes below 32 by trial (a thread per integer, most integers end there), the
+// others a thread per prime over its multiples in the tile from p^2 on, the
+// smallest kept by atomicMin.  Trial division of every integer by every prime up to
+// its root spent 3.36 ms at N = 10^7 on the few integers that need all of them;
+// this form takes 0.16 ms.
+constexpr uint32_t kSieveTile = 8192;
+constexpr uint32_t kTrialPrimes = 11;  // 2 .. 31
+
+__global__ void __launch_bounds__(kThreads) sieve_kernel(uint32_t* spf, uint32_t n, const uint32_t* primes,
+                                                         uint32_t nprimes) {
+    __shared__ uint32_t s[kSieveTile];
+    const uint32_t tiles = n / kSieveTile + 1;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t x0 = tile * kSieveTile, count = min(kSieveTile, n - x0 + 1);
+        for (uint32_t i = threadIdx.x; i < count; i += kThreads) {
+            const uint32_t x = x0 + i;
+            uint32_t f = x;  // spf[0] = 0, spf[1] = 1, spf[p] = p
+            for (uint32_t k = 0; k < kTrialPrimes && k < nprimes; ++k) {
+                const uint32_t p = primes[k];
+                if (p * p > x) break;
+                if (x % p == 0) {
+                    f = p;
+                    break;
+                }
             }
+            s[i] = f;
         }
-        spf[x] = s;
+        __syncthreads();
+        for (uint32_t k = kTrialPrimes + threadIdx.x; k < nprimes; k += kThreads) {
+            const uint32_t p = primes[k];
+            if (p * p >= x0 + count) break;  // (p <= sqrt(3e7): 32 bits)
+            uint32_t m = max(p * p, (x0 + p - 1) / p * p);
+            for (; m < x0 + count; m += p) atomicMin(&s[m - x0], p);
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < count; i += kThreads) spf[x0 + i] = s[i];
+        __syncthreads();
     }
 }
 
@@ -128,56 +150,84 @@ __device__ __forceinline__ uint32_t isqrt32(uint32_t r) {
     return v;
 }
 
-// A warp per integer p <= N; split primes only: the lanes try u = 1, 2, ...
-// 32 at a time for p - u^2 a square (the smallest such u, as the host), then
-// take the block's entries (a, r) in turn, each pi^r conj(pi)^(4a-r) by
-// repeated products (at most 4a <= 8 log_5 N of them, no per-thread arrays).
+// a b mod p for a, b < p < 2^32 by Barrett's reduction, inv = floor((2^64 - 1) / p):
+// the quotient is at most one short.
+__device__ __forceinline__ uint32_t mul_mod(uint32_t a, uint32_t b, uint32_t p, uint64_t inv) {
+    const uint64_t x = (uint64_t)a * b;
+    const uint64_t r = x - __umul64hi(x, inv) * p;
+    return (uint32_t)(r >= p ? r - p : r);
+}
+
+// The smaller u of p = u^2 + v^2 for every split prime p, left in pp_base[p],
+// by Cornacchia's method: r = a^((p - 1) / 4) is a square root of -1 for every
+// non-residue a (about every second one), and the first remainder of Euclid's
+// algorithm on (p, r) at or below sqrt(p) is one of the two.  A thread per
+// integer, bound by the chain of modular products on the one lane in 30 that has a
+// prime: 0.94 ms at N = 10^7 (2.77 ms with a 64-bit division per product).  With
+// pp_fill_kernel (1.06 ms) it replaces a search for u by a warp per prime (3.17 ms).
+__global__ void pp_root_kernel(const uint32_t* spf, uint32_t n, uint32_t* pp_base) {
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p <= n; p += gridDim.x * blockDim.x) {
+        if (!(p >= 5 && p % 4 == 1 && spf[p] == p)) continue;
+        uint32_t r = 0;
+        const uint64_t inv = ~0ull / p;
+        for (uint32_t a = 2; a < p; ++a) {
+            uint32_t base = a, e = (p - 1) / 4;
+            r = 1;
+            for (; e; e >>= 1) {
+                if (e & 1u) r = mul_mod(r, base, p, inv);
+                base = mul_mod(base, base, p, inv);
+            }
+            if (mul_mod(r, r, p, inv) == p - 1) break;
+        }
+        uint32_t x = p, y = r;
+        while ((uint64_t)y * y > p) {
+            const uint32_t t = x % y;
+            x = y;
+            y = t;
+        }
+        const uint32_t v = isqrt32(p - y * y);
+        pp_base[p] = min(y, v);
+    }
+}
+
+// A warp takes 32 integers at a time and, for each split prime p among them,
+// shares the block's entries (a, r): pi^r conj(pi)^(4a-r) by repeated products
+// (at most 4a <= 8 log_5 N of them, no per-thread arrays), pi = u + iv with the
+// u that pp_root_kernel left in pp_base.
 __global__ void pp_fill_kernel(const uint32_t* spf, uint32_t n, const uint64_t* offs, uint32_t* pp_base,
                                HotRec* pp_hot, __int128* pp_exact) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * blockDim.x / 32;
-    for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) / 32; p <= n; p += warps) {
-        if (!(p >= 5 && p % 4 == 1 && spf[p] == p)) {
-            if (lane == 0) pp_base[p] = 0xFFFFFFFFu;
-            continue;
-        }
-        uint32_t u = 0;
-        for (uint32_t u0 = 1; (uint64_t)u0 * u0 <= p; u0 += 32) {
-            const uint32_t uu = u0 + lane;
-            bool sq = false;
-            if ((uint64_t)uu * uu <= p) {
-                const uint32_t rem = p - uu * uu, v = isqrt32(rem);
-                sq = v * v == rem;
+    for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * 32; p0 <= n; p0 += warps * 32) {
+        const uint32_t mine = p0 + lane;
+        const bool split = mine <= n && mine >= 5 && mine % 4 == 1 && spf[mine] == mine;
+        const uint32_t root = split ? pp_base[mine] : 0u;
+        if (mine <= n) pp_base[mine] = split ? (uint32_t)offs[mine] : 0xFFFFFFFFu;
+        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, split); todo; todo &= todo - 1) {
+            const uint32_t src = __ffs(todo) - 1, p = p0 + src;
+            const uint32_t u = __shfl_sync(0xFFFFFFFFu, root, src), v = isqrt32(p - u * u);
+            const uint32_t max_a = 2 * power_count(p, n);
+            const uint64_t base = offs[p];
+            const Gauss pi{(__int128)u, (__int128)v}, pc{(__int128)u, -(__int128)v};
+            const uint32_t total = 2 * max_a * max_a + 3 * max_a;
+            for (uint32_t k = lane; k < total; k += 32) {
+                uint32_t a = 1, r = k;
+                while (r >= 4 * a + 1) {
+                    r -= 4 * a + 1;
+                    ++a;
+                }
+                Gauss val{1, 0};
+                for (uint32_t j = 0; j < r; ++j) val = gmul(val, pi);
+                for (uint32_t j = 0; j < 4 * a - r; ++j) val = gmul(val, pc);
+                pp_exact[2 * (base + k)] = val.re;
+                pp_exact[2 * (base + k) + 1] = val.im;
+                HotRec h;
+                h.re = i128_to_float(val.re);
+                h.im = i128_to_float(val.im);
+                h.rre = pack_residues(val.re) | (r == 2 * a ? kCentralBit : 0u);
+                h.rim = pack_residues(val.im);
+                pp_hot[base + k] = h;
             }
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, sq);
-            if (m) {
-                u = u0 + __ffs(m) - 1;
-                break;
-            }
-        }
-        const uint32_t v = isqrt32(p - u * u);
-        const uint32_t max_a = 2 * power_count(p, n);
-        const uint64_t base = offs[p];
-        if (lane == 0) pp_base[p] = (uint32_t)base;
-        const Gauss pi{(__int128)u, (__int128)v}, pc{(__int128)u, -(__int128)v};
-        const uint32_t total = 2 * max_a * max_a + 3 * max_a;
-        for (uint32_t k = lane; k < total; k += 32) {
-            uint32_t a = 1, r = k;
-            while (r >= 4 * a + 1) {
-                r -= 4 * a + 1;
-                ++a;
-            }
-            Gauss val{1, 0};
-            for (uint32_t j = 0; j < r; ++j) val = gmul(val, pi);
-            for (uint32_t j = 0; j < 4 * a - r; ++j) val = gmul(val, pc);
-            pp_exact[2 * (base + k)] = val.re;
-            pp_exact[2 * (base + k) + 1] = val.im;
-            HotRec h;
-            h.re = i128_to_float(val.re);
-            h.im = i128_to_float(val.im);
-            h.rre = pack_residues(val.re) | (r == 2 * a ? kCentralBit : 0u);
-            h.rim = pack_residues(val.im);
-            pp_hot[base + k] = h;
         }
     }
 }
@@ -215,29 +265,6 @@ __global__ void narrow_kernel(const uint64_t* in, uint32_t* out, uint32_t count)
         out[i] = (uint32_t)in[i];
 }
 
-struct Writer {
-    HotRec* hot;
-    ExactRec* exact;
-    uint32_t* owner;
-    uint32_t x;
-    uint64_t pos, end;  // end: the next segment's start
-    __device__ void emit(int64_t re, int64_t im, bool central) {
-        if (pos >= end) {  // more values than the segment holds: counted by the caller's check
-            ++pos;
-            return;
-        }
-        HotRec h;
-        h.re = (float)re;
-        h.im = (float)im;
-        h.rre = pack64(re) | (central ? kCentralBit : 0u);
-        h.rim = pack64(im);
-        hot[pos] = h;
-        exact[pos] = ExactRec{re, im};
-        owner[pos] = x;
-        ++pos;
-    }
-};
-
 __device__ __forceinline__ void cmul64(int64_t ar, int64_t ai, int64_t br, int64_t bi, int64_t& re, int64_t& im) {
     re = ar * br - ai * bi;
     im = ar * bi + ai * br;
@@ -246,55 +273,102 @@ __device__ __forceinline__ void cmul64(int64_t ar, int64_t ai, int64_t br, int64
 // Free set of x, then its central value: for the first non-central index i
 // and r_i < 2e_i, every digit combination of the later primes with the
 // earlier digit most significant (the host's recursion order).
-__global__ void seg_fill_kernel(const uint32_t* spf, uint32_t n, const uint32_t* seg_off, const uint32_t* pp_base,
-                                const __int128* pp_exact, HotRec* hot, ExactRec* exact, uint32_t* owner,
-                                unsigned int* err) {
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x <= n; x += gridDim.x * blockDim.x) {
-        if (x == 0) continue;
-        const Factors f = factor(spf, x);
-        Writer w{hot, exact, owner, x, seg_off[x], seg_off[x + 1]};
-        const __int128* vals[8];
-        uint32_t sizes[8];
-        for (uint32_t i = 0; i < f.count; ++i) {
-            vals[i] = pp_exact + 2 * ((uint64_t)pp_base[f.primes[i]] + pp_exponent_offset(f.exps[i]));
-            sizes[i] = 4u * f.exps[i] + 1;
-        }
-        int64_t prefix = (int64_t)f.fixed;  // fixed(x) * prod_{j<i} p_j^(2e_j)
-        for (uint32_t i = 0; i < f.count; ++i) {
-            const uint32_t centre = 2u * f.exps[i];
-            for (uint32_t r = 0; r < centre; ++r) {
-                // stack[j]: product through term j - 1; digits of terms i+1 .. count-1
-                int64_t sr[9], si[9];
-                uint32_t dig[8];
-                sr[i + 1] = prefix * (int64_t)vals[i][2 * r];
-                si[i + 1] = prefix * (int64_t)vals[i][2 * r + 1];
-                for (uint32_t j = i + 1; j < f.count; ++j) {
-                    dig[j] = 0;
-                    cmul64(sr[j], si[j], (int64_t)vals[j][0], (int64_t)vals[j][1], sr[j + 1], si[j + 1]);
+//
+// A CTA takes kFillRoots consecutive x: a thread factors each, then all threads
+// share the tile's records, one at a time and in order, so that the 36 bytes of a
+// record are written coalesced; a record's x is found among the tile's offsets,
+// its digits from its place in the segment.  (A thread per x that walked its own
+// segment took 10.7 ms at N = 10^7: 94.8 M records, stores of a warp to 32 segments; this
+// form takes 3.2 ms, 3.4 GB written.)
+constexpr uint32_t kFillRoots = 128;
+
+struct FillRoot {
+    uint64_t fixed;
+    uint32_t base[8];  // first prime-power value of the term
+    uint8_t e[8];
+    uint32_t count;
+    uint32_t pad;
+};
+
+__global__ void __launch_bounds__(kThreads) seg_fill_kernel(const uint32_t* spf, uint32_t n, const uint32_t* seg_off,
+                                                            const uint32_t* pp_base, const __int128* pp_exact,
+                                                            HotRec* hot, ExactRec* exact, uint32_t* owner,
+                                                            unsigned int* err) {
+    __shared__ FillRoot s_root[kFillRoots];
+    __shared__ uint32_t s_off[kFillRoots + 1];
+    const uint32_t tiles = n / kFillRoots + 1;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t x0 = tile * kFillRoots;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i <= kFillRoots; i += kThreads) s_off[i] = seg_off[min(x0 + i, n + 1)];
+        for (uint32_t i = threadIdx.x; i < kFillRoots; i += kThreads) {
+            const uint32_t x = x0 + i;
+            FillRoot r;
+            r.count = 0;
+            if (x >= 1 && x <= n) {
+                const Factors f = factor(spf, x);
+                uint32_t w = 1;
+                r.fixed = f.fixed;
+                r.count = f.count;
+                for (uint32_t j = 0; j < f.count; ++j) {
+                    r.base[j] = pp_base[f.primes[j]] + pp_exponent_offset(f.exps[j]);
+                    r.e[j] = (uint8_t)f.exps[j];
+                    w *= 4u * f.exps[j] + 1;
                 }
-                for (;;) {
-                    w.emit(sr[f.count], si[f.count], false);
-                    // advance the odometer, last digit fastest; done when every digit wrapped
-                    uint32_t j = f.count;
-                    bool more = false;
-                    while (j > i + 1) {
-                        --j;
-                        if (++dig[j] < sizes[j]) {
-                            more = true;
-                            break;
-                        }
-                        dig[j] = 0;
-                    }
-                    if (!more) break;
-                    for (uint32_t k = j; k < f.count; ++k)
-                        cmul64(sr[k], si[k], (int64_t)vals[k][2 * dig[k]], (int64_t)vals[k][2 * dig[k] + 1],
-                               sr[k + 1], si[k + 1]);
+                if (seg_off[x + 1] - seg_off[x] != (w - 1) / 2 + 1) atomicOr(err, 1u);  // segment size invariant
+            }
+            s_root[i] = r;
+        }
+        __syncthreads();
+        const uint32_t first = s_off[0], records = s_off[kFillRoots] - first;
+        for (uint32_t q = threadIdx.x; q < records; q += kThreads) {
+            const uint32_t pos = first + q;
+            uint32_t i = 0;  // the last root whose segment starts at or before pos
+#pragma unroll
+            for (uint32_t step = kFillRoots / 2; step; step >>= 1)
+                if (s_off[i + step] <= pos) i += step;
+            const FillRoot& R = s_root[i];
+            const uint32_t x = x0 + i, count = R.count;
+            uint32_t k = pos - s_off[i];
+            int64_t re = (int64_t)R.fixed, im = 0;
+            bool central = false;
+            uint32_t below = 1;  // values of the terms after the first non-central one
+            for (uint32_t j = 1; j < count; ++j) below *= 4u * R.e[j] + 1;
+            uint32_t t = 0;
+            for (;; ++t) {
+                if (t >= count) {
+                    central = true;
+                    break;
+                }
+                const uint32_t block = 2u * R.e[t] * below;
+                if (k < block) break;
+                k -= block;
+                re *= (int64_t)pp_exact[2 * ((uint64_t)R.base[t] + 2u * R.e[t])];  // p^(2e)
+                if (t + 1 < count) below /= 4u * R.e[t + 1] + 1;
+            }
+            if (central) {
+                re = (int64_t)x * x;
+            } else {
+                for (; t < count; ++t) {
+                    const uint32_t d = k / below;
+                    k -= d * below;
+                    if (t + 1 < count) below /= 4u * R.e[t + 1] + 1;
+                    const __int128* v = pp_exact + 2 * ((uint64_t)R.base[t] + d);
+                    int64_t nr, ni;
+                    cmul64(re, im, (int64_t)v[0], (int64_t)v[1], nr, ni);
+                    re = nr;
+                    im = ni;
                 }
             }
-            prefix *= (int64_t)vals[i][2 * centre];
+            HotRec h;
+            h.re = (float)re;
+            h.im = (float)im;
+            h.rre = pack64(re) | (central ? kCentralBit : 0u);
+            h.rim = pack64(im);
+            hot[pos] = h;
+            exact[pos] = ExactRec{re, im};
+            owner[pos] = x;
         }
-        w.emit((int64_t)x * (int64_t)x, 0, true);
-        if (w.pos != seg_off[x + 1]) atomicOr(err, 1u);  // segment size invariant
     }
 }
 
@@ -468,6 +542,8 @@ int build_device_cache(uint64_t n, int sm_count, CUstream_st* st, DeviceBuild* o
     DEV(dalloc(&b.pp_base, n + 1, &b.owned));
     DEV(dalloc(&b.pp_hot, pp_total, &b.owned));
     DEV(dalloc(&b.pp_exact, 2 * pp_total, &b.owned));
+    pp_root_kernel<<<grid, kThreads, 0, st>>>(b.spf, (uint32_t)n, b.pp_base);
+    DEV(cudaGetLastError());
     pp_fill_kernel<<<grid, kThreads, 0, st>>>(b.spf, (uint32_t)n, d_u64, b.pp_base, b.pp_hot, b.pp_exact);
     DEV(cudaGetLastError());
 
