@@ -38,8 +38,13 @@ constexpr uint32_t kDefaultItemTarget = 1u << 23;
 constexpr uint32_t kTileCap = 16384;           // largest m-range of one item
 constexpr uint32_t kTileMin = 32;
 constexpr uint32_t kBucketShift = 10;          // item ordering granularity in m
+constexpr uint64_t kArcLimit = 12000;          // the arc path from this limit on (see run_batched)
 constexpr uint64_t kMergedCap = 96ull << 20;   // shared-prime queue entries
 constexpr uint32_t kDescChunk = 1u << 24;       // shared-prime pairs set up per chunk (192 bytes each: 3 GB)
+// With the arc layout only the rest list's few pairs come by the shared-prime
+// kernels: small queues (0.5 GB; a plain scan enlarges them when it is called).
+constexpr uint64_t kArcMergedCap = 48ull << 20;
+constexpr uint32_t kArcDescChunk = 1u << 23;
 
 
 }  // namespace
@@ -132,7 +137,16 @@ int ensure_rows(hss_t* h, size_t rows) {
 }
 
 // Grows the shared-prime queue (entries of 16 bytes) to hold `n` pairs.
+// And a handle with the arc layout gets its whole chunk of descriptors here.
 int ensure_merged(hss_t* h, uint64_t n) {
+    if (n > h->desc_chunk && h->desc_chunk < kDescChunk) {
+        HSS_CUDA(h, cudaStreamSynchronize(h->stream));
+        uint4* larger = nullptr;
+        if (int s = device_alloc(h, &larger, (size_t)kDescChunk * kBigEntryWords)) return s;
+        device_free(h, h->d_desc);
+        h->d_desc = larger;
+        h->desc_chunk = kDescChunk;
+    }
     if (n <= h->merged_cap) return HSS_OK;
     if (n >= UINT32_MAX) return fail(h, HSS_ERR_OVERFLOW, "shared-prime queue beyond 32-bit indexing");
     HSS_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -188,6 +202,38 @@ int with_exact_retry(hss_t* h, Call call) {
     }
 }
 
+// Room for a launch group's rows, rest list and items (`bytes` in all) and
+// its rows' values; growing waits for the stream.
+int ensure_group(hss_t* h, size_t bytes, size_t values) {
+    if (bytes > h->group_cap) {
+        HSS_CUDA(h, cudaStreamSynchronize(h->stream));
+        device_free(h, h->d_group);
+        h->d_group = nullptr;
+        h->group_cap = 0;
+        const size_t cap = std::max(bytes + bytes / 4, (size_t)1 << 18);
+        if (int s = device_alloc(h, &h->d_group, cap)) return s;
+        for (unsigned char*& p : h->h_group) {
+            if (p) cudaFreeHost(p);
+            p = nullptr;
+            HSS_CUDA(h, cudaMallocHost(&p, cap));
+        }
+        h->group_cap = cap;
+    }
+    if (values > h->values_cap) {
+        HSS_CUDA(h, cudaStreamSynchronize(h->stream));
+        device_free(h, h->d_values);
+        device_free(h, h->d_value_hot);
+        h->d_values = nullptr;
+        h->d_value_hot = nullptr;
+        h->values_cap = 0;
+        const size_t cap = std::max(values + values / 4, (size_t)1 << 14);
+        if (int s = device_alloc(h, &h->d_values, cap)) return s;
+        if (int s = device_alloc(h, &h->d_value_hot, cap)) return s;
+        h->values_cap = cap;
+    }
+    return HSS_OK;
+}
+
 int ensure_items(hss_t* h, size_t n) {
     if (n > h->items_cap) {
         device_free(h, h->d_items);
@@ -213,9 +259,9 @@ int ensure_items(hss_t* h, size_t n) {
 // set over the same cache.
 int alloc_launch_buffers(hss_t* h) {
     h->hit_cap = h->opts.hit_capacity ? h->opts.hit_capacity : kDefaultHitCap;
-    h->merged_cap = (uint32_t)kMergedCap;
+    h->merged_cap = (uint32_t)(h->plan ? kArcMergedCap : kMergedCap);
     h->big_cap = 1u << 20;
-    h->desc_chunk = kDescChunk;
+    h->desc_chunk = h->plan ? kArcDescChunk : kDescChunk;
     h->exact_cap = h->opts.exact_capacity ? std::min<uint32_t>(h->opts.exact_capacity, 1u << 28) : 1u << 24;
     int s;
     if ((s = device_alloc(h, &h->d_hits, h->hit_cap)) || (s = device_alloc(h, &h->d_ctrl, 8)) ||
@@ -325,26 +371,31 @@ size_t build_items(hss_t* h, const RowRef* rows, size_t nrows, uint32_t* alpha_c
     return pos;
 }
 
-// Constants of the call's rows (row i of the call at index i).
-int upload_row_info(hss_t* h, const std::vector<uint64_t>& ls) {
-    if (ls.size() > h->row_info_cap) {
-        HSS_CUDA(h, cudaStreamSynchronize(h->stream));
-        device_free(h, h->d_row_info);
-        h->d_row_info = nullptr;
-        if (h->h_row_info) cudaFreeHost(h->h_row_info);
-        h->h_row_info = nullptr;
-        size_t cap = std::max(ls.size(), (size_t)1024);
-        int s = device_alloc(h, &h->d_row_info, cap);
-        if (s) return s;
-        HSS_CUDA(h, cudaMallocHost(&h->h_row_info, cap * sizeof(RowInfo)));
-        h->row_info_cap = cap;
-    }
+// Room for the constants of a call's rows; the stream is idle afterwards.
+int ensure_row_info(hss_t* h, size_t rows) {
     HSS_CUDA(h, cudaStreamSynchronize(h->stream));
-    for (size_t i = 0; i < ls.size(); ++i)
-        fill_row_info(h->spf.data(), h->seg_off.data(), h->limit, ls[i], &h->h_row_info[i]);
-    HSS_CUDA(h, cudaMemcpyAsync(h->d_row_info, h->h_row_info, ls.size() * sizeof(RowInfo), cudaMemcpyHostToDevice,
-                                h->stream));
-    h->h2d_bytes += ls.size() * sizeof(RowInfo);
+    if (rows <= h->row_info_cap) return HSS_OK;
+    device_free(h, h->d_row_info);
+    h->d_row_info = nullptr;
+    if (h->h_row_info) cudaFreeHost(h->h_row_info);
+    h->h_row_info = nullptr;
+    size_t cap = std::max(rows, (size_t)1024);
+    int s = device_alloc(h, &h->d_row_info, cap);
+    if (s) return s;
+    HSS_CUDA(h, cudaMallocHost(&h->h_row_info, cap * sizeof(RowInfo)));
+    h->row_info_cap = cap;
+    return HSS_OK;
+}
+
+// Constants of the call's rows first .. first + count - 1 (row i of the call,
+// root l_of(i), at index i).
+template <class LOf>
+int upload_row_info(hss_t* h, size_t first, size_t count, LOf l_of) {
+    for (size_t i = first; i < first + count; ++i)
+        fill_row_info(h->spf.data(), h->seg_off.data(), h->limit, l_of(i), &h->h_row_info[i]);
+    HSS_CUDA(h, cudaMemcpyAsync(h->d_row_info + first, h->h_row_info + first, count * sizeof(RowInfo),
+                                cudaMemcpyHostToDevice, h->stream));
+    h->h2d_bytes += count * sizeof(RowInfo);
     return HSS_OK;
 }
 
@@ -452,7 +503,9 @@ int run_batched_rows(hss_t* h, const RowRef* rows, size_t nrows) {
 }
 
 // Splits rows into groups whose shared-prime bound fits the queue.
-int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
+int run_products(hss_t* h, const std::vector<RowRef>& rows) {
+    if (int s = ensure_row_info(h, rows.size())) return s;
+    if (int s = upload_row_info(h, 0, rows.size(), [&](size_t i) { return rows[i].l; })) return s;
     size_t start = 0;
     while (start < rows.size()) {
         uint64_t bound = 0;
@@ -471,6 +524,107 @@ int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
     return HSS_OK;
 }
 
+// Launches the batched sequence for the rows collected in h->planner: reset
+// cursors and queues, rows and items H2D, the rows' values, the persistent
+// kernel, the shared-prime kernels over the rest list (when it holds any) and
+// the exact kernel.  Counters accumulate into d_rows[index].
+int run_planned(hss_t* h) {
+    // (an executable graph is updated in place only when it does not run)
+    if (h->opts.use_graph) HSS_CUDA(h, cudaStreamSynchronize(h->stream));
+    ArcPlanner& p = h->planner;
+    ArcConfig cfg;
+    cfg.threads = h->opts.block_threads == 512 ? 512 : 768;
+    cfg.ctas = h->sm_count * arc_max_ctas_per_sm(cfg.threads);
+    p.finish(*h->plan, (uint32_t)cfg.ctas, h->opts.item_target >> 10);
+    if (p.rows.empty()) return HSS_OK;
+    const size_t rows_b = p.rows.size() * sizeof(ArcRow), rest_b = p.rest.size() * sizeof(ArcRest),
+                 items_b = p.items.size() * sizeof(ArcItem);
+    auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t rest_at = align(rows_b), items_at = rest_at + align(rest_b), bytes = items_at + items_b;
+    if (int s = ensure_group(h, bytes, p.entries)) return s;
+    // the pinned buffer of two groups ago: its copy is done
+    const uint32_t turn = h->group_turn++ & 1u;
+    unsigned char* host = h->h_group[turn];
+    if (!h->group_copied[turn]) HSS_CUDA(h, cudaEventCreateWithFlags(&h->group_copied[turn], cudaEventDisableTiming));
+    if (!h->opts.use_graph) HSS_CUDA(h, cudaEventSynchronize(h->group_copied[turn]));
+    memcpy(host, p.rows.data(), rows_b);
+    if (rest_b) memcpy(host + rest_at, p.rest.data(), rest_b);
+    if (items_b) memcpy(host + items_at, p.items.data(), items_b);
+    ArcBuffers b{buffers(h, 0), reinterpret_cast<const ArcRow*>(h->d_group), h->d_values, h->d_value_hot, h->d_arc_tabs};
+    const ArcRest* rest = reinterpret_cast<const ArcRest*>(h->d_group + rest_at);
+    const ArcItem* items = reinterpret_cast<const ArcItem*>(h->d_group + items_at);
+    std::array<cudaEvent_t, 3> ev;
+    if (int e = take_events(h, &ev)) return e;
+    // Inside a capture the timing events become event-record nodes
+    // (cudaEventRecordExternal), so they still time the graph's kernels.
+    const unsigned int rec = h->opts.use_graph ? cudaEventRecordExternal : cudaEventRecordDefault;
+    uint32_t launched = 0;
+    auto enqueue = [&]() -> int {
+        HSS_CUDA(h, cudaMemcpyAsync(h->d_group, host, bytes, cudaMemcpyHostToDevice, h->stream));
+        if (!h->opts.use_graph) HSS_CUDA(h, cudaEventRecord(h->group_copied[turn], h->stream));
+        HSS_CUDA(h, cudaMemsetAsync(h->d_ctrl + 1, 0, 2 * sizeof(unsigned int), h->stream));
+        HSS_CUDA(h, cudaMemsetAsync(h->d_ctrl + 4, 0, 3 * sizeof(unsigned int), h->stream));
+        HSS_CUDA(h, cudaEventRecordWithFlags(ev[0], h->stream, rec));
+        HSS_CUDA(h, launch_arc_values(h->dev, (uint32_t)p.rows.size(), b, h->stream));
+        HSS_CUDA(h, launch_arc(h->dev, items, (uint32_t)p.items.size(), cfg, b, h->stream));
+        HSS_CUDA(h, cudaEventRecordWithFlags(ev[1], h->stream, rec));
+        launched = 3;  // values, persistent, exact
+        if (!p.rest.empty()) {
+            uint32_t merged = 0;
+            HSS_CUDA(h, launch_arc_rest(h->dev, rest, (uint32_t)p.rest.size(), b, h->sm_count * 8, h->stream));
+            HSS_CUDA(h, launch_merged(h->dev, p.rest_pairs, b, h->sm_count * 4, h->stream, &merged));
+            launched += 1 + merged;
+        }
+        HSS_CUDA(h, launch_arc_exact(h->dev, b, h->sm_count * 4, h->stream));
+        HSS_CUDA(h, cudaEventRecordWithFlags(ev[2], h->stream, rec));
+        return HSS_OK;
+    };
+    if (h->opts.use_graph) {
+        if (int e = run_captured(h, enqueue)) return e;
+    } else if (int e = enqueue()) {
+        return e;
+    }
+    h->h2d_bytes += bytes;
+    h->marks.push_back(ev);
+    h->launches += launched;
+    return HSS_OK;
+}
+
+// Splits the call's rows into launch groups whose values and rest pairs fit the
+// buffers.  Of a long call the first eighth is a group by itself, so that the
+// device works while the host plans the rest.
+constexpr uint64_t kGroupValues = 8ull << 20;
+constexpr size_t kGroupRows = 1u << 20;
+constexpr size_t kLongCall = 2048;
+
+// Below kArcLimit the product kernel stays the faster path: class lists are too
+// short there for runs to pay (roots 80..4979 at LIMIT 5000: 3.3 ms by
+// products, 4.3 ms by arcs; 1..3000 at 3000: 1.5 and 2.3; 8000..9999 at 10^4: 1.5
+// and 1.3; 5000..7000 at 20,000: 10.6 and 6.1).
+int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
+    if (!h->plan) return run_products(h, rows);
+    h->planner.clear();
+    size_t start = 0;
+    if (int s = ensure_row_info(h, rows.size())) return s;
+    while (start < rows.size()) {
+        const size_t piece = start == 0 && rows.size() >= kLongCall && !h->opts.use_graph ? rows.size() / 8 : rows.size() - start;
+        if (int s = upload_row_info(h, start, piece, [&](size_t i) { return rows[i].l; })) return s;
+        for (size_t i = start; i < start + piece; ++i) {
+            h->planner.add(h->h_row_info[i], rows[i].index, h->limit, h->dev.max_exponent, 1, h->limit,
+                           min_roots(h->limit, rows.size()));
+            const bool full = h->planner.entries >= kGroupValues || h->planner.rows.size() >= kGroupRows ||
+                              h->planner.rest_pairs >= h->merged_cap / 2;
+            if (!full && i + 1 < start + piece) continue;
+            if (h->planner.rest_pairs > h->merged_cap)
+                if (int s = ensure_merged(h, h->planner.rest_pairs)) return s;
+            if (int s = run_planned(h)) return s;
+            h->planner.clear();
+        }
+        start += piece;
+    }
+    return HSS_OK;
+}
+
 int run_plain(hss_t* h, uint64_t first, uint64_t last) {
     for (uint64_t b = first; b <= last; b += kPlainBatch) {
         uint32_t nrows = (uint32_t)std::min<uint64_t>(kPlainBatch, last - b + 1);
@@ -480,10 +634,7 @@ int run_plain(hss_t* h, uint64_t first, uint64_t last) {
             bound += merged_bound(h, l);
             acap = std::max(acap, free_count(h, l) + 1);
         }
-        if (bound > h->merged_cap) {
-            int g = ensure_merged(h, bound);
-            if (g) return g;
-        }
+        if (int g = ensure_merged(h, bound)) return g;
         HSS_CUDA(h, cudaMemsetAsync(h->d_ctrl + 1, 0, sizeof(unsigned int), h->stream));
         HSS_CUDA(h, cudaMemsetAsync(h->d_ctrl + 4, 0, 3 * sizeof(unsigned int), h->stream));
         LaunchBuffers buf = buffers(h, b - first);
@@ -587,6 +738,30 @@ void copy_hits(const std::vector<DevHit>& in, hss_hit* out, uint32_t cap) {
     }
 }
 
+// The arc layout of the handle's cache (h->dev, h->records), enqueued on the stream.
+int open_arc_layout(hss_t* h) {
+    if (h->limit < kArcLimit) return HSS_OK;
+    auto plan = std::make_shared<ArcPlan>();
+    ArcBuild b;
+    std::string err;
+    int s = plan_arc_blocks(h->dev.seg_off, h->limit, h->stream, plan.get(), &err);
+    if (!s) s = build_arc_layout(h->dev, h->records, *plan, h->stream, &b, &err);
+    if (s) return fail(h, s, err);
+    h->allocations.insert(h->allocations.end(), b.owned.begin(), b.owned.end());
+    h->dev.blocks = b.blocks;
+    for (uint32_t f = 0; f < kFields; ++f) h->dev.arc_w[f] = b.w[f];
+    h->dev.arc_ang = b.ang;
+    h->dev.arc_part = b.part;
+    h->dev.arc_src = b.src;
+    h->dev.arc_m = b.m;
+    h->dev.arc_xy = b.xy;
+    h->dev.arc_index = b.index;
+    h->dev.pos = b.pos;
+    h->dev.block_cap = plan->cap;
+    h->plan = std::move(plan);
+    return HSS_OK;
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ exports
@@ -687,15 +862,29 @@ int hss_open(uint64_t limit, int device, const hss_opts* opts, hss_t** out) {
     }
     h->sm_count = prop.multiProcessorCount;
     int s = HSS_OK;
+    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+        delete h;
+        return HSS_ERR_CUDA;
+    }
     if (!h->opts.host_build) {
         // the cache built by kernels on the device (same arrays and values as the host build)
-        if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
-            delete h;
-            return HSS_ERR_CUDA;
-        }
         DeviceBuild db;
         std::string err;
-        s = build_device_cache(limit, h->sm_count, h->stream, &db, &err);
+        auto take = [&] {
+            h->records = db.records;
+            h->dev.limit = limit;
+            h->dev.spf = db.spf;
+            h->dev.seg_off = db.seg_off;
+            h->dev.hot = db.hot;
+            h->dev.exact = db.exact;
+            h->dev.owner = db.owner;
+            h->dev.pp_base = db.pp_base;
+            h->dev.pp_hot = db.pp_hot;
+            h->dev.pp_exact = db.pp_exact;
+            h->dev.max_exponent = db.max_exponent;
+            return open_arc_layout(h);
+        };
+        s = build_device_cache(limit, h->sm_count, h->stream, &db, &err, take);
         if (s) {
             hss_close(h);
             return s;
@@ -705,20 +894,9 @@ int hss_open(uint64_t limit, int device, const hss_opts* opts, hss_t** out) {
             hss_close(h);
             return HSS_ERR_LIMIT;
         }
-        h->records = db.records;
         h->ref_flattened = db.reference_flattened;
         h->ref_cached = db.reference_cached;
         h->prep_seconds = db.seconds;
-        h->dev.limit = limit;
-        h->dev.spf = db.spf;
-        h->dev.seg_off = db.seg_off;
-        h->dev.hot = db.hot;
-        h->dev.exact = db.exact;
-        h->dev.owner = db.owner;
-        h->dev.pp_base = db.pp_base;
-        h->dev.pp_hot = db.pp_hot;
-        h->dev.pp_exact = db.pp_exact;
-        h->dev.max_exponent = db.max_exponent;
         h->seg_off = std::move(db.seg_off_host);
         h->spf = std::move(db.spf_host);
     } else {
@@ -728,13 +906,13 @@ int hss_open(uint64_t limit, int device, const hss_opts* opts, hss_t** out) {
         int threads = h->opts.prep_threads ? (int)h->opts.prep_threads : (int)(hw ? hw : 1);
         s = build_host_cache(limit, threads, &hc, &err);
         if (s) {
-            delete h;
+            hss_close(h);
             return s;
         }
         uint32_t longest = 0;
         for (uint64_t x = 1; x <= limit; ++x) longest = std::max(longest, hc.seg_off[x + 1] - hc.seg_off[x]);
         if (longest > kItemRecords) {
-            delete h;
+            hss_close(h);
             return HSS_ERR_LIMIT;
         }
         h->records = hc.records;
@@ -767,10 +945,18 @@ int hss_open(uint64_t limit, int device, const hss_opts* opts, hss_t** out) {
         h->dev.max_exponent = hc.max_exponent;
         h->seg_off = std::move(hc.seg_off);
         h->spf = std::move(hc.spf);
+        if (cudaDeviceSynchronize() != cudaSuccess || (s = open_arc_layout(h)) ||
+            cudaStreamSynchronize(h->stream) != cudaSuccess) {
+            hss_close(h);
+            return s ? s : HSS_ERR_CUDA;
+        }
     }
     std::vector<uint8_t> tables(kTableTotalBytes);
     build_residue_tables(tables.data());
-    if ((s = upload(h, &h->d_tables, tables.data(), kTableTotalBytes)) || (s = alloc_launch_buffers(h))) {
+    std::vector<uint8_t> arc_tabs(kArcTabBytes);
+    build_arc_tables(arc_tabs.data());
+    if ((s = upload(h, &h->d_tables, tables.data(), kTableTotalBytes)) ||
+        (s = upload(h, &h->d_arc_tabs, arc_tabs.data(), kArcTabBytes)) || (s = alloc_launch_buffers(h))) {
         hss_close(h);
         return s;
     }
@@ -787,6 +973,10 @@ void hss_close(hss_t* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void* p : h->allocations) cudaFree(p);
     if (h->h_items) cudaFreeHost(h->h_items);
+    for (unsigned char* p : h->h_group)
+        if (p) cudaFreeHost(p);
+    for (cudaEvent_t e : h->group_copied)
+        if (e) cudaEventDestroy(e);
     if (h->h_rows) cudaFreeHost(h->h_rows);
     if (h->h_row_info) cudaFreeHost(h->h_row_info);
     if (h->h_ctrl) cudaFreeHost(h->h_ctrl);
@@ -863,12 +1053,8 @@ int search_locked(hss_t* h, uint64_t first, uint64_t last, int mode, hss_counts*
     const size_t rows = (size_t)(last - first + 1);
     int s = begin_call(h, rows);
     if (s) return s;
-    {
-        std::vector<uint64_t> ls(rows);
-        for (size_t r = 0; r < rows; ++r) ls[r] = first + r;
-        if ((s = upload_row_info(h, ls))) return s;
-    }
     if (mode == HSS_MODE_PLAIN) {
+        if ((s = ensure_row_info(h, rows)) || (s = upload_row_info(h, 0, rows, [&](size_t i) { return first + i; }))) return s;
         s = run_plain(h, first, last);
     } else {
         std::vector<RowRef> refs(rows);
@@ -967,15 +1153,9 @@ int search_many_locked(hss_t* h, const uint64_t* firsts, const uint64_t* lasts, 
     int s = begin_call(h, rows);
     if (s) return s;
     std::vector<RowRef> refs;
-    std::vector<uint64_t> ls;
     refs.reserve(rows);
-    ls.reserve(rows);
     for (uint32_t i = 0; i < count; ++i)
-        for (uint64_t l = firsts[i]; l <= lasts[i]; ++l) {
-            refs.push_back(RowRef{l, (uint32_t)refs.size()});
-            ls.push_back(l);
-        }
-    if ((s = upload_row_info(h, ls))) return s;
+        for (uint64_t l = firsts[i]; l <= lasts[i]; ++l) refs.push_back(RowRef{l, (uint32_t)refs.size()});
     if ((s = run_batched(h, refs))) return s;
     std::vector<DevHit> found;
     uint32_t nfound = 0;
@@ -1073,6 +1253,8 @@ hss_t* make_lane(hss_t* h, int* status) {
     lane->spf = h->spf;
     lane->dev = h->dev;
     lane->d_tables = h->d_tables;
+    lane->d_arc_tabs = h->d_arc_tabs;
+    lane->plan = h->plan;
     int s = alloc_launch_buffers(lane);
     if (!s && cudaMallocHost(&lane->h_ctrl, 8 * sizeof(unsigned int)) != cudaSuccess) s = HSS_ERR_MEMORY;
     if (s) {
@@ -1106,9 +1288,7 @@ int launch_wave(hss_t* h, hss_t* lane, const Wave& w) {
     const size_t n = w.rows.size();
     int s = begin_call(lane, n);
     if (s) return s;
-    std::vector<uint64_t> ls(n);
-    for (size_t i = 0; i < n; ++i) ls[i] = w.rows[i].l;
-    if ((s = upload_row_info(lane, ls)) || (s = ensure_slots(lane, n))) return s;
+    if ((s = ensure_slots(lane, n))) return s;
     for (size_t i = 0; i < n; ++i) lane->h_slots[i] = w.owner[i]->slot + (uint32_t)(w.rows[i].l - w.owner[i]->first);
     HSS_CUDA(lane, cudaMemcpyAsync(lane->d_slots, lane->h_slots, n * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                    lane->stream));

@@ -6,6 +6,7 @@
 #include <condition_variable>
 #include <deque>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -13,6 +14,7 @@
 
 #include "hss_api_status.h"
 #include "hss_kernels.h"
+#include "hss_plan.h"
 
 namespace hss {
 struct Request;
@@ -93,10 +95,25 @@ struct hss_ctx {
     uint4* d_merged = nullptr;
     uint32_t merged_cap = 0;
     uint8_t* d_tables = nullptr;
+
     hss::WorkItem* d_items = nullptr;
     size_t items_cap = 0;
     hss::WorkItem* h_items = nullptr;  // pinned
     size_t h_items_cap = 0;
+    // arc path: the block plan (shared with the serving lanes), the planner of
+    // a launch group, its rows, rest list and items in one buffer (device and
+    // pinned staging), and the rows' values
+    std::shared_ptr<const hss::ArcPlan> plan;
+    hss::ArcPlanner planner;
+    uint8_t* d_arc_tabs = nullptr;
+    unsigned char* d_group = nullptr;
+    unsigned char* h_group[2] = {nullptr, nullptr};      // pinned; groups alternate, so one is planned
+    cudaEvent_t group_copied[2] = {nullptr, nullptr};    // while the other's copy may still run
+    uint32_t group_turn = 0;
+    size_t group_cap = 0;
+    hss::ArcValue* d_values = nullptr;
+    hss::HotRec* d_value_hot = nullptr;
+    size_t values_cap = 0;
     hss::RowCounts* h_rows = nullptr;  // pinned
     size_t h_rows_cap = 0;
     hss::RowInfo* d_row_info = nullptr;  // constants of the call's rows

@@ -462,7 +462,8 @@ cudaError_t dalloc(T** p, size_t count, std::vector<void*>* owned) {
 
 }  // namespace
 
-int build_device_cache(uint64_t n, int sm_count, CUstream_st* st, DeviceBuild* out, std::string* err) {
+int build_device_cache(uint64_t n, int sm_count, CUstream_st* st, DeviceBuild* out, std::string* err,
+                       const std::function<int()>& on_records) {
     auto t0 = std::chrono::steady_clock::now();
     if (n < 1 || n > kMaxLimit) {
         *err = "limit out of range";
@@ -524,6 +525,7 @@ int build_device_cache(uint64_t n, int sm_count, CUstream_st* st, DeviceBuild* o
     DEV(dalloc(&b.spf, n + 1, &b.owned));
     sieve_kernel<<<grid, kThreads, 0, st>>>(b.spf, (uint32_t)n, d_primes, (uint32_t)small_primes.size());
     DEV(cudaGetLastError());
+    b.spf_host.resize(n + 1);  // (while the device works; the pages are touched here)
 
     // 2. prime-power table
     pp_size_kernel<<<grid, kThreads, 0, st>>>(b.spf, (uint32_t)n, d_u64, d_flags + 0);
@@ -546,6 +548,8 @@ int build_device_cache(uint64_t n, int sm_count, CUstream_st* st, DeviceBuild* o
     DEV(cudaGetLastError());
     pp_fill_kernel<<<grid, kThreads, 0, st>>>(b.spf, (uint32_t)n, d_u64, b.pp_base, b.pp_hot, b.pp_exact);
     DEV(cudaGetLastError());
+
+    b.seg_off_host.resize(n + 2);
 
     // 3. segment offsets
     seg_size_kernel<<<grid, kThreads, 0, st>>>(b.spf, (uint32_t)n, d_u64, d_refc, d_flags + 1);
@@ -579,9 +583,13 @@ int build_device_cache(uint64_t n, int sm_count, CUstream_st* st, DeviceBuild* o
                                                b.owner, d_flags + 2);
     DEV(cudaGetLastError());
 
+    if (on_records)
+        if (int s = on_records()) {
+            cudaStreamSynchronize(st);
+            release();
+            return s;
+        }
     // host copies the item builder reads
-    b.spf_host.resize(n + 1);
-    b.seg_off_host.resize(n + 2);
     DEV(cudaMemcpyAsync(b.spf_host.data(), b.spf, (n + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DEV(cudaMemcpyAsync(b.seg_off_host.data(), b.seg_off, (n + 2) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DEV(cudaMemcpyAsync(flags, d_flags, sizeof flags, cudaMemcpyDeviceToHost, st));

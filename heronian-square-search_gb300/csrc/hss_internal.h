@@ -21,6 +21,7 @@
 // both coordinates' residues modulo 9360 and 45917 packed in one word.
 #pragma once
 #include <stdint.h>
+#include <vector_types.h>
 
 #ifdef __CUDACC__
 #define HSS_HD __host__ __device__
@@ -114,6 +115,80 @@ struct DevHit {
 };
 static_assert(sizeof(DevHit) == 48, "hit record is 48 bytes");
 
+// Filter moduli of the arc path (hss_arc.cuh): three residue fields below
+// 2^10, each the product of two primes, so that a value's (re, im) and its
+// root's m^4 fit one 32-bit word per field.
+constexpr uint32_t kFields = 3;
+constexpr uint32_t kFieldMod[kFields] = {17 * 37, 13 * 61, 11 * 73};
+HSS_HD constexpr uint32_t field_mod(uint32_t f) { return f == 0 ? 17 * 37 : f == 1 ? 13 * 61 : 11 * 73; }
+// ceil(2^32 / M): multiplying by it maps t mod M to the top bits of a word
+HSS_HD constexpr uint32_t field_scale(uint32_t f) { return 0xFFFFFFFFu / field_mod(f) + 1u; }
+
+// Roots m by divisibility: 3 classes by powers of two (odd, 2 mod 4, 0 mod 4)
+// times divisibility by 3 and by 5.
+constexpr uint32_t kTypes = 12;
+HSS_HD inline uint32_t type_of(uint32_t m) {
+    const uint32_t v = (m & 1u) ? 0u : (m & 3u) ? 1u : 2u;
+    return v * 4u + (m % 3u == 0 ? 2u : 0u) + (m % 5u == 0 ? 1u : 0u);
+}
+
+// The roots of a type repeat with period 60: their residues in 1..60 order,
+// and how many of them are at most r, for r = 0..59.
+struct TypeTables {
+    uint8_t count[kTypes];
+    uint8_t res[kTypes][16];
+    uint8_t upto[kTypes][60];
+};
+constexpr TypeTables make_type_tables() {
+    TypeTables t{};
+    for (uint32_t x = 1; x <= 60; ++x) {
+        const uint32_t v = (x & 1u) ? 0u : (x & 3u) ? 1u : 2u;
+        const uint32_t ty = v * 4u + (x % 3u == 0 ? 2u : 0u) + (x % 5u == 0 ? 1u : 0u);
+        t.res[ty][t.count[ty]++] = (uint8_t)x;
+        if (x < 60)
+            for (uint32_t k = 0; k < kTypes; ++k) t.upto[k][x] = t.count[k];
+    }
+    return t;
+}
+// The root of a given rank (from 0) among those of its type, and the number of
+// them up to x.
+HSS_HD inline uint32_t nth_root(const TypeTables& t, uint32_t type, uint32_t rank) {
+    const uint32_t c = t.count[type];
+    return 60u * (rank / c) + t.res[type][rank % c];
+}
+HSS_HD inline uint32_t roots_upto(const TypeTables& t, uint32_t type, uint32_t x) {
+    return x / 60u * t.count[type] + t.upto[type][x % 60u];
+}
+
+// One block of the arc layout: the records of consecutive roots of one type,
+// sorted by (class list, angle).  List s < 8 holds the non-central values of
+// class s = s8 << 2 | b3 << 1 | b5 (see hss_blocks.cu), list 8 the central
+// values by root.
+constexpr uint32_t kLists = 9;
+constexpr uint32_t kBlockEntries = 6144;  // at most: what fits beside 24 warps' own shared memory
+struct ArcBlock {
+    uint32_t base;             // first entry in the sorted arrays (a multiple of 16)
+    uint32_t n;                // entries, central ones included
+    uint32_t m_lo, m_hi;       // smallest and largest root
+    uint32_t n_m, n_plain;     // roots, and those without a split prime
+    uint32_t type;
+    uint32_t rank0;            // rank of m_lo among the roots of its type
+    uint16_t list[kLists + 1]; // start of each list; list[9] = n
+    uint16_t pad[2];
+    uint32_t pad2[2];
+};
+static_assert(sizeof(ArcBlock) == 64, "block record is 64 bytes");
+
+// A block's roots in kParts ranges of equal length (the window bounds of a row
+// are kept per range): range of root m.
+constexpr uint32_t kParts = 32;
+HSS_HD inline uint32_t part_step(uint32_t m_lo, uint32_t m_hi) { return (m_hi - m_lo) / kParts + 1; }
+
+// Index of a block's lists by angle: entry (list, x) is the first entry of the
+// list whose angle is at least x << kBucketShift (x = 0 .. kBuckets).
+constexpr uint32_t kBucketShift = 25, kBuckets = 64;
+constexpr uint32_t kIndexWords = 8 * (kBuckets + 2) / 2;  // 16-bit entries, two per word
+
 // Device-resident factor cache for one limit N (all pointers are device
 // pointers; host mirrors of seg_off / spf are kept by the owner).
 struct DeviceCache {
@@ -127,6 +202,19 @@ struct DeviceCache {
     const HotRec* pp_hot;       // prime-power values, hot form
     const __int128* pp_exact;   // prime-power values, exact (re, im) pairs
     uint32_t max_exponent;      // largest exponent covered by the prime-power table
+    // arc layout (hss_blocks.cu): blocks, and per sorted entry the three
+    // residue words (re | im << 10 | m^4 << 20 of one field), the angle and
+    // the record it comes from; pos: a record's place in its block
+    const ArcBlock* blocks;
+    const uint32_t* arc_index;  // kIndexWords per block
+    const uint32_t* arc_w[kFields];
+    const uint32_t* arc_ang;
+    const uint8_t* arc_part;    // which of its block's kParts root ranges the entry's root is in
+    const uint32_t* arc_src;
+    const uint32_t* arc_m;      // the entry's root
+    const float2* arc_xy;       // its value (positive imaginary part)
+    const uint16_t* pos;
+    uint32_t block_cap;         // entries of the largest block
 };
 
 // Offset of exponent e's 4e+1 values within prime p's block:

@@ -39,6 +39,7 @@
 // thread per pair, in chunks of the queue) and run by merged_kernel (a warp
 // per pair) or, when their lists exceed a warp's slice, merged_big_kernel (a
 // CTA per pair).
+#include <type_traits>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
@@ -1943,11 +1944,15 @@ __global__ void __launch_bounds__(kMergedThreads, 4) merged_big_kernel(const Dev
     }
 }
 
+#include "hss_arc.cuh"
+
 // Exact work queued by the search kernels (rare: products whose window
 // decision was within the float error bound, and possible hits).  Exact
 // coordinates come from the cache (row values doubled) or, for pairs that
-// share a split prime, from the two term groups rebuilt for the pair.
-__global__ void __launch_bounds__(128) exact_kernel(const DeviceCache cache, const LaunchBuffers buf) {
+// share a split prime, from the two term groups rebuilt for the pair.  Terms of
+// arc rows only come to the form with ArcBuffers.
+template <class Buffers>
+__global__ void __launch_bounds__(128) exact_kernel(const DeviceCache cache, const Buffers buf) {
     __shared__ __align__(16) uint8_t s_tab[kTableBytes];
     for (uint32_t i = threadIdx.x; i < kTableBytes; i += blockDim.x) s_tab[i] = buf.tables[i];
     __syncthreads();
@@ -1955,6 +1960,23 @@ __global__ void __launch_bounds__(128) exact_kernel(const DeviceCache cache, con
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const ExactItem it = buf.exact_queue[i];
         const uint32_t kind = it.kind & 3u, p = (it.kind >> 2) & 1u, o = (it.kind >> 3) & 1u;
+        if constexpr (std::is_same_v<Buffers, ArcBuffers>) {
+            if (it.kind & 32u) {  // one term of an arc row
+                uint32_t c = 0, r = 0;
+                arc_exact_term(cache, buf, it, s_tab, &c, &r);
+                if (kind != kExHit) {
+                    RowCounts* rc = &buf.rows[it.row];
+                    atomicAdd(&rc->candidates, (unsigned long long)c);
+                    atomicAdd(&rc->r16, (unsigned long long)r);
+                    atomicAdd(&rc->exact, 1ull);
+                    if (buf.arc_rows[it.arc_row].p != 1) {
+                        atomicAdd(&rc->mcandidates, (unsigned long long)c);
+                        atomicAdd(&rc->mr16, (unsigned long long)r);
+                    }
+                }
+                continue;
+            }
+        }
         const bool shared_prime = (it.kind & 16u) != 0;
         i128 ar, ai, br, bi;
         if (shared_prime) {
@@ -2051,8 +2073,8 @@ void fill_row_info(const uint32_t* spf, const uint32_t* seg_off, uint64_t n, uin
     R->l2 = l * l;
     R->l4 = (u128)R->l2 * R->l2;
     R->n4 = (u128)(n * n) * (n * n);
-    R->lmodA = mod_u128_small(R->l4, kModA);
-    R->lmodD = mod_u128_small(R->l4, kModD);
+    R->lmodA = pow4_mod((uint32_t)(l % kModA), kModA);
+    R->lmodD = pow4_mod((uint32_t)(l % kModD), kModD);
     R->l2x2f = (float)(2 * R->l2);
     R->l4f = (float)R->l4;
     R->l2modA = (uint32_t)(R->l2 % kModA);
@@ -2112,6 +2134,62 @@ void build_residue_tables(uint8_t* out) {
     for (uint32_t z = 0; z < 2 * kModD; ++z)
         if ((words[(z % kModD) >> 5] >> ((z % kModD) & 31u)) & 1u) words2[z >> 5] |= 1u << (z & 31u);
     memcpy(wide + kTabD2, words2, sizeof words2);
+}
+
+void build_arc_tables(uint8_t* out) {
+    memset(out, 0, kArcTabBytes);
+    for (uint32_t f = 0; f < kFields; ++f) {
+        const uint32_t M = field_mod(f), K = field_scale(f);
+        const int64_t delta = (int64_t)((uint64_t)K * M - (1ull << 32));
+        // the filter's sum is K t mod 2^32 with t = r mod M in [-2 M^2, 3 M^2 + M]:
+        // K r + delta q for t = r + M q
+        const int64_t q0 = -2 * (int64_t)M - 1, q1 = 3 * (int64_t)M + 1;
+        bool is4[1024] = {};
+        for (uint64_t x = 0; x < M; ++x) is4[x * x % M * x % M * x % M] = true;
+        for (uint32_t r = 0; r < M; ++r) {
+            if (!is4[r]) continue;
+            const int64_t lo = ((int64_t)K * r + delta * q0) >> 21, hi = ((int64_t)K * r + delta * q1) >> 21;
+            for (int64_t x = lo; x <= hi; ++x) out[(f << 11) + (uint32_t)(x & 2047)] = 1;
+        }
+    }
+}
+
+// One CTA per SM: 24 warps (the default) or 16.
+static const void* arc_fn(int threads) {
+    return threads == 512 ? (const void*)arc_kernel<512> : (const void*)arc_kernel<768>;
+}
+
+static size_t arc_smem_bytes(int threads) { return threads == 512 ? sizeof(ArcSmem<16>) : sizeof(ArcSmem<24>); }
+
+int arc_max_ctas_per_sm(int threads) {
+    const void* fn = arc_fn(threads);
+    const size_t smem = arc_smem_bytes(threads);
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess) return 1;
+    return n > 0 ? n : 1;
+}
+
+cudaError_t launch_arc_values(const DeviceCache& cache, uint32_t n_rows, const ArcBuffers& buf,
+                              cudaStream_t stream) {
+    if (n_rows) arc_value_kernel<<<n_rows, 64, 0, stream>>>(cache, buf);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_arc(const DeviceCache& cache, const ArcItem* items, uint32_t n_items, const ArcConfig& cfg,
+                       const ArcBuffers& buf, cudaStream_t stream) {
+    const size_t smem = arc_smem_bytes(cfg.threads);
+    const void* fn = arc_fn(cfg.threads);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    void* args[] = {(void*)&cache, (void*)&items, (void*)&n_items, (void*)&buf};
+    return cudaLaunchKernel(fn, dim3(cfg.ctas), dim3(cfg.threads), args, smem, stream);
+}
+
+cudaError_t launch_arc_rest(const DeviceCache& cache, const ArcRest* rest, uint32_t n, const LaunchBuffers& buf,
+                            int ctas, cudaStream_t stream) {
+    if (n) arc_rest_kernel<<<n < (uint32_t)ctas ? n : (uint32_t)ctas, 128, 0, stream>>>(cache, rest, n, buf);
+    return cudaGetLastError();
 }
 
 size_t batched_smem_bytes(int threads, uint32_t alpha_cap) {
@@ -2201,7 +2279,12 @@ cudaError_t launch_scatter_rows(const RowCounts* rows, const uint32_t* slots, ui
 }
 
 cudaError_t launch_exact(const DeviceCache& cache, const LaunchBuffers& buf, int ctas, cudaStream_t stream) {
-    exact_kernel<<<ctas, 128, 0, stream>>>(cache, buf);
+    exact_kernel<LaunchBuffers><<<ctas, 128, 0, stream>>>(cache, buf);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_arc_exact(const DeviceCache& cache, const ArcBuffers& buf, int ctas, cudaStream_t stream) {
+    exact_kernel<ArcBuffers><<<ctas, 128, 0, stream>>>(cache, buf);
     return cudaGetLastError();
 }
 

@@ -49,10 +49,66 @@ struct RowInfo {
 // Exact work queued by the search kernels for exact_kernel: kind bits 0-1
 // (0: count a whole product, 1: count one orientation, 2: hit test of one
 // orientation), bit 2: product alpha*conj(beta), bit 3: orientation (y, x),
-// bit 4: shared-prime pair (a, b are list entries rather than cache indices).
+// bit 4: shared-prime pair (a, b are list entries rather than cache indices),
+// bit 5: one term of an arc row (a: entry of the row's values, b: record of
+// m', arc_row and variant: the row and which of the value's eight forms).
 struct ExactItem {
-    uint32_t kind, a, b, l, m, row, pad0, pad1;
+    uint32_t kind, a, b, l, m, row, arc_row, variant;
 };
+
+// A row of the arc path: root l (RowInfo `row`) against the roots m = P m',
+// m' in [m_lo, m_hi], where P is a product of powers of l's split primes and
+// m' is prime to them.  P = 1 covers the pairs without a common split prime;
+// the others cover the pairs whose common part is exactly P, as l P against m'.
+struct ArcRow {
+    uint32_t row, p;
+    uint32_t m_lo, m_hi;       // range of m'
+    uint32_t ent, na;          // first entry of its values (free set of l P, then the central value) and their number
+    uint32_t cc_hi;            // largest m' with l^4 + m^4 <= N^4 (0: none)
+    uint32_t l;
+    uint32_t c0[kFields];      // field_scale * (l^4 mod M)
+    uint32_t c3[kFields];      // field_scale * (P^4 mod M)
+    float q0;                  // l^2 / (2 P^2): the window's upper cosine times m'^2
+    float zscale;              // 2 l^2 P^2: |gamma beta| / m'^2
+    float lw_hi, lw_lo;        // l^4 - N^4 in two floats
+    uint32_t l_class;          // 0 odd, 1 = 2 mod 4, 2 = 0 mod 4; + 4 if 3 | l; + 8 if 5 | l
+    uint32_t pad;
+};
+static_assert(sizeof(ArcRow) == 80, "arc row is 80 bytes");
+
+// One unit of arc work: rows v0 .. v0 + nv - 1 (one l_class parity and the
+// same divisibility by 3 and 5) against one block.  Warps take whole rows,
+// except for the first `split` rows (those of many values), whose groups of
+// 32 runs are shared by `parts` warps each; where an item has too few rows for
+// its warps even so, `share` warps take every share-th run of a group.
+struct ArcItem {
+    uint32_t block, base;         // the block and its first entry
+    uint32_t v0;
+    uint16_t nv, split, parts, n; // n: the block's entries
+    uint32_t share;               // 1, 2, 4 or 8
+};
+static_assert(sizeof(ArcItem) == 24, "arc item is 24 bytes");
+
+struct ArcConfig {
+    int threads;      // CTA size (512 or 768)
+    int ctas;         // persistent grid size
+};
+
+// Shared-prime pairs too few for a row of their own: (l, P m') for m' in
+// [m_lo, m_hi], handed to the shared-prime queue.
+struct ArcRest {
+    uint32_t row, l, p, m_lo, m_hi;
+};
+
+// Row-side value of the arc path (one per conjugate pair; the kernel forms
+// its conjugate and its products with i, -1, -i): argument, class bits and
+// the filter residues times field_scale.
+struct __align__(16) ArcValue {
+    uint32_t ang;              // argument, 2^32 / (2 pi) units
+    uint32_t cls;              // s8 << 2 | b3 << 1 | b5
+    uint32_t re[kFields], im[kFields];
+};
+static_assert(sizeof(ArcValue) == 32, "arc value is 32 bytes");
 
 // 16-byte words of one big_queue entry.
 constexpr uint32_t kBigEntryWords = 12;
@@ -84,6 +140,31 @@ struct LaunchBuffers {
     unsigned int* exact_count;
     uint32_t exact_cap;
 };
+
+// The same and a group's arc rows (apart, since some kernels keep a copy of
+// their buffers on the stack).
+struct ArcBuffers : LaunchBuffers {
+    const ArcRow* arc_rows;     // rows of the arc path
+    ArcValue* arc_values;       // their values, and the same as hot records (doubled)
+    HotRec* arc_hot;
+    const uint8_t* arc_tabs;    // kArcTabBytes filter tables
+};
+
+// Filter tables of the arc path: per field 2048 bytes, byte x 1 when some
+// fourth-power residue r mod M can give the top 11 bits x.
+constexpr uint32_t kArcTabBytes = kFields << 11;
+void build_arc_tables(uint8_t* out /* kArcTabBytes */);
+
+int arc_max_ctas_per_sm(int threads);
+
+// Values of the arc rows (one CTA per row).
+cudaError_t launch_arc_values(const DeviceCache& cache, uint32_t n_rows, const ArcBuffers& buf, cudaStream_t stream);
+// Persistent kernel over the arc items.
+cudaError_t launch_arc(const DeviceCache& cache, const ArcItem* items, uint32_t n_items, const ArcConfig& cfg,
+                       const ArcBuffers& buf, cudaStream_t stream);
+// The pairs of the rest list that are not skipped, into the shared-prime queue.
+cudaError_t launch_arc_rest(const DeviceCache& cache, const ArcRest* rest, uint32_t n, const LaunchBuffers& buf,
+                            int ctas, cudaStream_t stream);
 
 // Host-side fill of a RowInfo from the smallest-prime-factor table.
 void fill_row_info(const uint32_t* spf, const uint32_t* seg_off, uint64_t limit, uint64_t l, RowInfo* out);
@@ -126,6 +207,8 @@ double int32_peak_ops(int device, int sm_count, double* ms);
 
 // Exact work queued by the search kernels; run after them.
 cudaError_t launch_exact(const DeviceCache& cache, const LaunchBuffers& buf, int ctas, cudaStream_t stream);
+// The same for a queue that may hold terms of arc rows.
+cudaError_t launch_arc_exact(const DeviceCache& cache, const ArcBuffers& buf, int ctas, cudaStream_t stream);
 
 // Serving: copies a wave's row counters rows[i] into the requests' device-
 // resident state, state[slots[i]], marked done (RowCounts::pad = 1), so a

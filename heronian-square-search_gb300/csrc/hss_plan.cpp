@@ -1,0 +1,212 @@
+// hss_plan.cpp - rows and work items of the arc path (host side).
+#include "hss_plan.h"
+
+#include <math.h>
+
+#include <algorithm>
+
+namespace hss {
+namespace {
+
+using u128 = unsigned __int128;
+using i128 = __int128;
+
+uint64_t fourth_root(u128 x) {
+    uint64_t r = (uint64_t)sqrt(sqrt((double)x));
+    while (r > 0 && (u128)r * r * r * r > x) --r;
+    while ((u128)(r + 1) * (r + 1) * (r + 1) * (r + 1) <= x) ++r;
+    return r;
+}
+
+}  // namespace
+
+// A row (l, P) costs its value list and a visit to every block of its range; the
+// shared-prime kernels set every pair up by itself, and cost three launches
+// that wait for one another.  Few rows: no shared-prime launch at all (37 roots at
+// LIMIT 10^7 1.8 ms against 2.2 ms with 48 roots, one at 70,000 0.21 against 0.28 ms).
+// Many: 48 (512 roots at 10^7 114.5 ms, against 117 ms with 1 and 114.4 with 150), at small
+// limits, whose blocks hold fewer roots each, 150 (2,001 roots at 20,000 6.1 ms against 6.9 ms with 48).
+uint64_t min_roots(uint64_t limit, size_t rows) { return rows <= 64 ? 1 : limit < 1000000 ? 150 : 48; }
+
+void ArcPlanner::clear() {
+    rows.clear();
+    rest.clear();
+    items.clear();
+    keys.clear();
+    entries = rest_pairs = 0;
+}
+
+void ArcPlanner::add(const RowInfo& R, uint32_t row, uint64_t limit, uint32_t max_exponent, uint64_t m0, uint64_t m1,
+                     uint64_t least) {
+    const uint64_t l = R.l;
+    m0 = std::max(m0, l);
+    m1 = std::min(m1, limit);
+    if (m0 > m1) return;
+    const uint64_t zero_hi = R.n4 > R.l4 ? fourth_root(R.n4 - R.l4) : 0;  // largest m with w <= 0
+    const i128 lw = (i128)R.l4 - (i128)R.n4;
+    const float lw_hi = i128_to_float(lw), lw_lo = i128_to_float(lw - (i128)lw_hi);
+    uint32_t c0[kFields];
+    for (uint32_t f = 0; f < kFields; ++f) {
+        const uint32_t M = field_mod(f), r = (uint32_t)(l % M), r2 = r * r % M;
+        c0[f] = field_scale(f) * (r2 * r2 % M);
+    }
+    const uint32_t l_class = ((l & 1) ? 0u : (l & 3) ? 1u : 2u) | (R.l3 ? 4u : 0u) | (R.l5 ? 8u : 0u);
+    // every P, depth first over the split primes: (P, number of values, prime)
+    struct Part {
+        uint64_t p, w;
+        uint32_t i;
+        bool fits;
+    };
+    Part stack[64];
+    int top = 0;
+    stack[top++] = Part{1, 2ull * R.free_l + 1, 0, true};
+    while (top) {
+        const Part s = stack[--top];
+        if (s.i < R.nsplit) {
+            const uint64_t p = R.sp[s.i], e = R.se[s.i];
+            stack[top++] = Part{s.p, s.w, s.i + 1, s.fits};
+            uint64_t q = s.p;
+            for (uint64_t a = 1; q <= limit / p; ++a) {
+                q *= p;
+                if (q > m1) break;
+                // no room for a multiple of q in [m0, m1] does not exclude a
+                // further power: every q <= m1 is visited
+                stack[top++] = Part{q, s.w / (4 * e + 1) * (4 * (e + a) + 1), s.i + 1, s.fits && e + a <= max_exponent};
+            }
+            continue;
+        }
+        const uint64_t lo = (m0 + s.p - 1) / s.p, hi = m1 / s.p;
+        if (lo > hi) continue;
+        if (s.p != 1 && (!s.fits || hi - lo + 1 < least)) {
+            rest.push_back(ArcRest{row, (uint32_t)l, (uint32_t)s.p, (uint32_t)lo, (uint32_t)hi});
+            rest_pairs += hi - lo + 1;
+            continue;
+        }
+        ArcRow a{};
+        a.row = row;
+        a.p = (uint32_t)s.p;
+        a.m_lo = (uint32_t)lo;
+        a.m_hi = (uint32_t)hi;
+        a.na = (uint32_t)((s.w + 1) / 2);
+        a.cc_hi = (uint32_t)(zero_hi / s.p);
+        a.l = (uint32_t)l;
+        const double p2 = (double)s.p * (double)s.p, l2 = (double)R.l2;
+        a.q0 = (float)(l2 / (2.0 * p2));
+        a.zscale = (float)(2.0 * l2 * p2);
+        a.lw_hi = lw_hi;
+        a.lw_lo = lw_lo;
+        a.l_class = l_class;
+        for (uint32_t f = 0; f < kFields; ++f) {
+            const uint32_t M = field_mod(f), p1 = (uint32_t)s.p % M, p2m = p1 * p1 % M;
+            a.c0[f] = c0[f];
+            a.c3[f] = field_scale(f) * (p2m * p2m % M);
+        }
+        entries += a.na;
+        keys.push_back((uint64_t)s.p << 3 | ((l_class & 3) ? 4u : 0u) | (R.l3 ? 2u : 0u) | (R.l5 ? 1u : 0u));
+        rows.push_back(a);
+    }
+}
+
+void ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target) {
+    items.clear();
+    if (rows.empty()) return;
+    // rows by (P, parity, divisibility by 3 and 5), those of many values first
+    struct Order {
+        uint64_t key, rest;  // rest: values descending, then the order of addition
+    };
+    std::vector<Order> order(rows.size());
+    for (size_t i = 0; i < rows.size(); ++i) order[i] = Order{keys[i], (uint64_t)(UINT32_MAX - rows[i].na) << 32 | i};
+    std::sort(order.begin(), order.end(),
+              [](const Order& x, const Order& y) { return x.key != y.key ? x.key < y.key : x.rest < y.rest; });
+    std::vector<ArcRow> sorted(rows.size());
+    uint32_t ent = 0;
+    for (size_t i = 0; i < order.size(); ++i) {
+        sorted[i] = rows[(uint32_t)order[i].rest];
+        keys[i] = order[i].key;
+        sorted[i].ent = ent;
+        ent += sorted[i].na;
+    }
+    rows.swap(sorted);
+    // the blocks of a type whose roots meet [lo, hi]
+    auto range_of = [&](uint32_t t, uint32_t lo, uint32_t hi, uint32_t* b0, uint32_t* b1) {
+        const uint32_t end = plan.type_first[t + 1];
+        const uint32_t* start = plan.start[t].data();
+        uint32_t x = start[lo >> plan.start_shift], y;
+        while (x < end && plan.blocks[x].m_hi < lo) ++x;
+        y = std::max(x, start[hi >> plan.start_shift]);
+        while (y < end && plan.blocks[y].m_lo <= hi) ++y;
+        *b0 = x;
+        *b1 = y;
+    };
+    auto type_allowed = [](uint64_t key, uint32_t t) {
+        return !((key & 4u) && t >= 4) && !((key & 2u) && (t & 2u)) && !((key & 1u) && (t & 1u));
+    };
+    auto cost = [](const ArcRow& r) { return (uint64_t)r.na + 16; };
+    struct Group {
+        size_t g0, g1;
+        uint32_t b0[kTypes], b1[kTypes];  // its blocks of every type
+    };
+    std::vector<Group> groups;
+    uint64_t total = 0;
+    for (size_t g0 = 0; g0 < rows.size();) {
+        size_t g1 = g0;
+        uint64_t w = 0;
+        uint32_t lo = rows[g0].m_lo, hi = 0;
+        while (g1 < rows.size() && keys[g1] == keys[g0]) {
+            w += cost(rows[g1]);
+            lo = std::min(lo, rows[g1].m_lo);
+            hi = std::max(hi, rows[g1].m_hi);
+            ++g1;
+        }
+        Group g{};
+        g.g0 = g0;
+        g.g1 = g1;
+        for (uint32_t t = 0; t < kTypes; ++t) {
+            if (!type_allowed(keys[g0], t)) continue;
+            range_of(t, lo, hi, &g.b0[t], &g.b1[t]);
+            total += w * (g.b1[t] - g.b0[t]);
+        }
+        groups.push_back(g);
+        g0 = g1;
+    }
+    // item size: the caller's, or about twelve items per resident CTA
+    const uint64_t target = std::max<uint64_t>(16, item_target ? item_target : total / ((uint64_t)ctas * 12));
+    std::vector<ArcItem> cut;  // the group's chunks of rows, without a block
+    std::vector<uint32_t> cut_lo;
+    for (const Group& g : groups) {
+        cut.clear();
+        cut_lo.clear();
+        for (size_t i = g.g0; i < g.g1;) {
+            uint64_t w = 0;
+            size_t e = i;
+            uint32_t lo = UINT32_MAX;
+            for (; e < g.g1 && e - i < 512 && (e == i || w + cost(rows[e]) <= target); ++e) {
+                w += cost(rows[e]);
+                lo = std::min(lo, rows[e].m_lo);
+            }
+            // rows above a forty-eighth of the chunk are shared by warps
+            uint32_t split = 0;
+            while (i + split < e && cost(rows[i + split]) * 48 > w) ++split;
+            // (a part holds at least a few groups of 32 runs)
+            const uint64_t parts =
+                split ? std::max<uint64_t>(1, std::min({(uint64_t)24, (cost(rows[i]) * 48 + w - 1) / w, (uint64_t)rows[i].na / 2})) : 1;
+            cut.push_back(ArcItem{0, 0, (uint32_t)i, (uint16_t)(e - i), (uint16_t)split, (uint16_t)parts, 0, 1});
+            // fewer units than warps: the runs of a group are shared too
+            uint64_t units = split * parts + (e - i - split);
+            for (; units < 16 && cut.back().share < 8; units *= 2) cut.back().share *= 2;
+            cut_lo.push_back(lo);
+            i = e;
+        }
+        for (uint32_t t = 0; t < kTypes; ++t)
+            for (uint32_t b = g.b0[t]; b < g.b1[t]; ++b)
+                for (size_t c = 0; c < cut.size(); ++c) {
+                    if (cut_lo[c] > plan.blocks[b].m_hi) continue;
+                    items.push_back(cut[c]);
+                    items.back().block = b;
+                    items.back().base = plan.blocks[b].base;
+                    items.back().n = (uint16_t)plan.blocks[b].n;
+                }
+    }
+}
+
+}  // namespace hss

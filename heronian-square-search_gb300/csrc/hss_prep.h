@@ -3,6 +3,7 @@
 #include <stdint.h>
 
 #include <memory>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -69,7 +70,9 @@ struct DeviceBuild {
 };
 
 // Builds the cache for limit N on the current device, on `stream`, with grids
-// of sm_count * 8 CTAs.  Returns 0 or a negative hss status with *err set.
-int build_device_cache(uint64_t limit, int sm_count, CUstream_st* stream, DeviceBuild* out, std::string* err);
+// of sm_count * 8 CTAs.  on_records (when given) is called once the records are
+// enqueued (further kernels on the stream that read them).  Returns 0 or a negative hss status with *err set.
+int build_device_cache(uint64_t limit, int sm_count, CUstream_st* stream, DeviceBuild* out, std::string* err,
+                       const std::function<int()>& on_records = {});
 
 }  // namespace hss
