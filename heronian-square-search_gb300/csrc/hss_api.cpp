@@ -535,7 +535,7 @@ int run_planned(hss_t* h) {
     ArcConfig cfg;
     cfg.threads = h->opts.block_threads == 512 ? 512 : 768;
     cfg.ctas = h->sm_count * arc_max_ctas_per_sm(cfg.threads);
-    p.finish(*h->plan, (uint32_t)cfg.ctas, h->opts.item_target >> 10);
+    if (!p.finish(*h->plan, (uint32_t)cfg.ctas, h->opts.item_target >> 10)) return HSS_ERR_MEMORY;
     if (p.rows.empty()) return HSS_OK;
     const size_t rows_b = p.rows.size() * sizeof(ArcRow), rest_b = p.rest.size() * sizeof(ArcRest),
                  items_b = p.items.size() * sizeof(ArcItem);

@@ -6,13 +6,14 @@
 // cannot allow that at search time: processes whose device memory is owned by
 // a pool or an embedding runtime fixed at start-up, or loops that cannot take
 // the implicit synchronisation an allocation brings.  hss_search_noalloc runs
-// the same batched launch sequence (persistent kernel, shared-prime kernels,
-// exact kernel) with all per-call device scratch in one file-scope array of
+// the same batched launch sequence (by arcs where the handle has their layout: 8
+// rows at LIMIT 10^7 took 29.6 ms by products and take 5.0 ms; else the product,
+// shared-prime and exact kernels) with all per-call device scratch in one file-scope array of
 // kNoAllocBytes that is part of the library image, and host staging in static
 // buffers.  Every GPU that loads the library holds the array until the process
 // exits.  The array bounds the work of one launch, not the call: a call whose
-// rows have more shared-prime pairs than the array holds runs as several
-// launch groups, and a group whose exact-work queue fills runs again in
+// rows have more values or shared-prime pairs than the array holds runs as several
+// launches or launch groups, and a group whose exact-work queue fills runs again in
 // smaller pieces.
 //
 // Set-up: the array's name is a host-side stand-in, not a device address.
@@ -30,6 +31,7 @@
 
 #include "hss_ctx.h"
 #include "hss_kernels.h"
+#include "hss_plan.h"
 #include "hss_prep.h"
 
 namespace {
@@ -58,6 +60,17 @@ constexpr size_t kOffDesc = align256(kOffBig + (size_t)kNaBig * kBigEntryWords *
 constexpr size_t kOffExact = align256(kOffDesc + (size_t)kNaDesc * kBigEntryWords * sizeof(uint4));
 constexpr size_t kNoAllocBytes = align256(kOffExact + kNaExact * sizeof(ExactItem));
 static_assert(kNoAllocBytes <= (24u << 20), "scratch stays within 24 MiB");
+
+// With the arc layout the space of the items, the shared-prime queues and their
+// descriptors holds arc rows, their values and the arc items instead.
+constexpr uint32_t kNaArcRows = 8192;
+constexpr uint32_t kNaArcValues = 1u << 18;
+constexpr uint32_t kNaArcItems = 1u << 18;
+constexpr size_t kOffArcRows = kOffItems;
+constexpr size_t kOffArcValues = align256(kOffArcRows + kNaArcRows * sizeof(ArcRow));
+constexpr size_t kOffArcHot = align256(kOffArcValues + (size_t)kNaArcValues * sizeof(ArcValue));
+constexpr size_t kOffArcItems = align256(kOffArcHot + (size_t)kNaArcValues * sizeof(HotRec));
+static_assert(kOffArcItems + (size_t)kNaArcItems * sizeof(ArcItem) <= kOffExact, "the arc arrays end before the exact queue");
 
 static __device__ __align__(256) unsigned char g_scratch[kNoAllocBytes];
 
@@ -129,6 +142,7 @@ uint64_t shared_bound(const hss_t* h, uint64_t l, uint64_t m0, uint64_t m1) {
 // halved by m-range), so the limits bound memory, not the interval.
 struct Piece {
     uint32_t r, m0, m1;
+    bool products;  // by the product kernels (the handle has no arc layout, or the piece's rows outgrow the arc arrays)
 };
 constexpr uint32_t kNaPieces = 4096;  // pending pieces (a depth-first work stack)
 constexpr uint32_t kNaMinSpan = 64;   // a piece is not halved below this many roots
@@ -141,28 +155,8 @@ struct GroupResult {
     uint64_t h2d, d2h;
 };
 
-// Runs pieces g_stack[lo, hi) as one launch group, adding its row counters to
-// g_host_sum and its hits to g_host_hits[*nh ...] (at most kNaHits kept,
-// *found counts them all).  Returns HSS_ERR_OVERFLOW, with nothing added, when
-// a queue of the scratch overflowed.
-int run_group(hss_t* h, unsigned char* base, uint32_t rows, uint32_t lo, uint32_t hi, uint32_t alpha_cap,
-              uint32_t* nh, uint64_t* found, GroupResult* res) {
-    const uint32_t npieces = hi - lo;
-    const uint32_t per_piece = kNaItems / npieces;
-    uint32_t n_items = 0;
-    uint64_t shared = 0;
-    for (uint32_t i = lo; i < hi; ++i) {
-        const Piece& pc = g_stack[i];
-        const uint64_t l = g_host_rows[pc.r].l;
-        shared += shared_bound(h, l, pc.m0, pc.m1);
-        const uint64_t span = pc.m1 - pc.m0;
-        const uint64_t parts = std::max<uint64_t>(1, std::min<uint64_t>(per_piece, (span + 31) / 32));
-        const uint64_t tile = (span + parts - 1) / parts;
-        for (uint64_t m = pc.m0; m < pc.m1; m += tile)
-            g_host_items[n_items++] =
-                WorkItem{(uint32_t)l, (uint32_t)m, (uint32_t)std::min<uint64_t>(m + tile, pc.m1), pc.r};
-    }
-
+// The scratch array as launch buffers.
+LaunchBuffers scratch_buffers(const hss_t* h, unsigned char* base) {
     LaunchBuffers b;
     unsigned int* ctrl = reinterpret_cast<unsigned int*>(base + kOffCtrl);
     b.rows = reinterpret_cast<RowCounts*>(base + kOffRows);
@@ -186,25 +180,13 @@ int run_group(hss_t* h, unsigned char* base, uint32_t rows, uint32_t lo, uint32_
     b.exact_cap = kNaExact;
     b.tables = h->d_tables;
     b.row_info = reinterpret_cast<const RowInfo*>(base + kOffRowInfo);
+    return b;
+}
 
+// Waits for a launch group and adds its row counters and hits to the call's.
+int collect(hss_t* h, const LaunchBuffers& b, uint32_t rows, uint32_t* nh, uint64_t* found, GroupResult* res) {
     cudaStream_t st = h->stream;
-    NA_CUDA(cudaMemsetAsync(base + kOffCtrl, 0, kNaCtrl * sizeof(unsigned int), st));
-    NA_CUDA(cudaMemsetAsync(base + kOffRows, 0, rows * sizeof(RowCounts), st));
-    NA_CUDA(cudaMemcpyAsync(base + kOffItems, g_host_items, n_items * sizeof(WorkItem), cudaMemcpyHostToDevice, st));
-    BatchedConfig cfg;
-    cfg.threads = h->opts.block_threads ? (int)h->opts.block_threads : 256;
-    cfg.min_blocks =
-        h->opts.ctas_per_sm ? (int)h->opts.ctas_per_sm : (cfg.threads == 128 ? 4 : cfg.threads == 512 ? 1 : 2);
-    cfg.alpha_cap = alpha_cap;
-    cfg.ctas = h->sm_count * batched_max_ctas_per_sm(cfg.threads, cfg.min_blocks,
-                                                     batched_smem_bytes(cfg.threads, alpha_cap));
-    NA_CUDA(cudaEventRecord(h->ev0, st));
-    NA_CUDA(launch_batched(h->dev, reinterpret_cast<const WorkItem*>(base + kOffItems), n_items, cfg, b, st));
-    uint32_t merged_launches = 0;
-    NA_CUDA(launch_merged(h->dev, shared, b, h->sm_count * 4, st, &merged_launches));
-    NA_CUDA(launch_exact(h->dev, b, h->sm_count * 4, st));
-    NA_CUDA(cudaEventRecord(h->ev1, st));
-    NA_CUDA(cudaMemcpyAsync(g_host_ctrl, ctrl, sizeof g_host_ctrl, cudaMemcpyDeviceToHost, st));
+    NA_CUDA(cudaMemcpyAsync(g_host_ctrl, b.hit_count, sizeof g_host_ctrl, cudaMemcpyDeviceToHost, st));
     NA_CUDA(cudaMemcpyAsync(g_host_counts, b.rows, rows * sizeof(RowCounts), cudaMemcpyDeviceToHost, st));
     NA_CUDA(cudaStreamSynchronize(st));
     if (g_host_ctrl[3] & ~15u) return fail(h, HSS_ERR_CUDA, "hss_search_noalloc: a device index check failed");
@@ -229,10 +211,118 @@ int run_group(hss_t* h, unsigned char* base, uint32_t rows, uint32_t lo, uint32_
         a.mcandidates += c.mcandidates;
         a.mr16 += c.mr16;
     }
-    res->launches = 2 + merged_launches;
-    res->h2d = n_items * sizeof(WorkItem);
     res->d2h = sizeof g_host_ctrl + rows * sizeof(RowCounts) + take * sizeof(DevHit);
     return HSS_OK;
+}
+
+// Runs pieces g_stack[lo, hi) as one launch group, adding its row counters to
+// g_host_sum and its hits to g_host_hits[*nh ...] (at most kNaHits kept,
+// *found counts them all).  Returns HSS_ERR_OVERFLOW, with nothing added, when
+// a queue of the scratch overflowed.
+int run_group(hss_t* h, unsigned char* base, uint32_t rows, uint32_t lo, uint32_t hi, uint32_t alpha_cap,
+              uint32_t* nh, uint64_t* found, GroupResult* res) {
+    const uint32_t npieces = hi - lo;
+    const uint32_t per_piece = kNaItems / npieces;
+    uint32_t n_items = 0;
+    uint64_t shared = 0;
+    for (uint32_t i = lo; i < hi; ++i) {
+        const Piece& pc = g_stack[i];
+        const uint64_t l = g_host_rows[pc.r].l;
+        shared += shared_bound(h, l, pc.m0, pc.m1);
+        const uint64_t span = pc.m1 - pc.m0;
+        const uint64_t parts = std::max<uint64_t>(1, std::min<uint64_t>(per_piece, (span + 31) / 32));
+        const uint64_t tile = (span + parts - 1) / parts;
+        for (uint64_t m = pc.m0; m < pc.m1; m += tile)
+            g_host_items[n_items++] =
+                WorkItem{(uint32_t)l, (uint32_t)m, (uint32_t)std::min<uint64_t>(m + tile, pc.m1), pc.r};
+    }
+
+    LaunchBuffers b = scratch_buffers(h, base);
+    cudaStream_t st = h->stream;
+    NA_CUDA(cudaMemsetAsync(base + kOffCtrl, 0, kNaCtrl * sizeof(unsigned int), st));
+    NA_CUDA(cudaMemsetAsync(base + kOffRows, 0, rows * sizeof(RowCounts), st));
+    NA_CUDA(cudaMemcpyAsync(base + kOffItems, g_host_items, n_items * sizeof(WorkItem), cudaMemcpyHostToDevice, st));
+    BatchedConfig cfg;
+    cfg.threads = h->opts.block_threads ? (int)h->opts.block_threads : 256;
+    cfg.min_blocks =
+        h->opts.ctas_per_sm ? (int)h->opts.ctas_per_sm : (cfg.threads == 128 ? 4 : cfg.threads == 512 ? 1 : 2);
+    cfg.alpha_cap = alpha_cap;
+    cfg.ctas = h->sm_count * batched_max_ctas_per_sm(cfg.threads, cfg.min_blocks,
+                                                     batched_smem_bytes(cfg.threads, alpha_cap));
+    NA_CUDA(cudaEventRecord(h->ev0, st));
+    NA_CUDA(launch_batched(h->dev, reinterpret_cast<const WorkItem*>(base + kOffItems), n_items, cfg, b, st));
+    uint32_t merged_launches = 0;
+    NA_CUDA(launch_merged(h->dev, shared, b, h->sm_count * 4, st, &merged_launches));
+    NA_CUDA(launch_exact(h->dev, b, h->sm_count * 4, st));
+    NA_CUDA(cudaEventRecord(h->ev1, st));
+    if (int s = collect(h, b, rows, nh, found, res)) return s;
+    res->launches = 2 + merged_launches;
+    res->h2d = n_items * sizeof(WorkItem);
+    return HSS_OK;
+}
+
+// The same by arcs: the pieces' rows (l, P), in launches of as many rows as
+// the arc arrays hold (a row of a call of at most 64 roots is never left to the
+// shared-prime kernels, so their queues stay empty).  kNoRoom, with nothing
+// added, when the rows outgrow the host's table or one row the values' array.
+constexpr int kNoRoom = 1;
+constexpr uint32_t kNaPlanRows = 1u << 15;
+ArcPlanner::Arena<kNaPlanRows, 1> g_plan_arena;
+ArcPlanner::Arena<kNaArcRows, kNaArcItems> g_launch_arena;
+ArcPlanner g_plan, g_launch;
+
+int run_arc_group(hss_t* h, unsigned char* base, uint32_t rows, uint32_t lo, uint32_t hi, uint32_t* nh, uint64_t* found,
+                  GroupResult* res) {
+    g_plan.use(g_plan_arena);
+    g_launch.use(g_launch_arena);
+    g_plan.clear();
+    for (uint32_t i = lo; i < hi; ++i) {
+        const Piece& pc = g_stack[i];
+        g_plan.add(g_host_rows[pc.r], pc.r, h->limit, h->dev.max_exponent, pc.m0, pc.m1 - 1, 1);
+    }
+    if (g_plan.rows.over() || g_plan.rest_pairs) return kNoRoom;
+    g_plan.sort();
+    ArcBuffers b{scratch_buffers(h, base), reinterpret_cast<const ArcRow*>(base + kOffArcRows),
+                 reinterpret_cast<ArcValue*>(base + kOffArcValues), reinterpret_cast<HotRec*>(base + kOffArcHot),
+                 h->d_arc_tabs};
+    const ArcItem* items = reinterpret_cast<const ArcItem*>(base + kOffArcItems);
+    ArcConfig cfg;
+    cfg.threads = h->opts.block_threads == 512 ? 512 : 768;
+    cfg.ctas = h->sm_count * arc_max_ctas_per_sm(cfg.threads);
+    cudaStream_t st = h->stream;
+    NA_CUDA(cudaMemsetAsync(base + kOffCtrl, 0, kNaCtrl * sizeof(unsigned int), st));
+    NA_CUDA(cudaMemsetAsync(base + kOffRows, 0, rows * sizeof(RowCounts), st));
+    NA_CUDA(cudaEventRecord(h->ev0, st));
+    const size_t all = g_plan.rows.size();
+    for (size_t i0 = 0; i0 < all;) {
+        size_t i1 = i0;
+        uint64_t values = 0;
+        while (i1 < all && i1 - i0 < kNaArcRows && values + g_plan.rows[i1].na <= kNaArcValues) values += g_plan.rows[i1++].na;
+        // the host arrays may still be read by the last launch's copies
+        if (i0) NA_CUDA(cudaStreamSynchronize(st));
+        for (; i1 > i0; i1 = i0 + (i1 - i0) / 2) {
+            g_launch.take(g_plan, i0, i1);
+            if (g_launch.finish(*h->plan, (uint32_t)cfg.ctas, h->opts.item_target >> 10)) break;
+        }
+        if (i1 == i0) {
+            NA_CUDA(cudaStreamSynchronize(st));
+            return kNoRoom;
+        }
+        const size_t rows_b = g_launch.rows.size() * sizeof(ArcRow), items_b = g_launch.items.size() * sizeof(ArcItem);
+        NA_CUDA(cudaMemcpyAsync(base + kOffArcRows, g_launch.rows.data(), rows_b, cudaMemcpyHostToDevice, st));
+        if (items_b)
+            NA_CUDA(cudaMemcpyAsync(base + kOffArcItems, g_launch.items.data(), items_b, cudaMemcpyHostToDevice, st));
+        NA_CUDA(cudaMemsetAsync(b.next_item, 0, sizeof(unsigned int), st));
+        NA_CUDA(cudaMemsetAsync(b.exact_count, 0, sizeof(unsigned int), st));
+        NA_CUDA(launch_arc_values(h->dev, (uint32_t)g_launch.rows.size(), b, st));
+        NA_CUDA(launch_arc(h->dev, items, (uint32_t)g_launch.items.size(), cfg, b, st));
+        NA_CUDA(launch_arc_exact(h->dev, b, h->sm_count * 4, st));
+        res->launches += 3;
+        res->h2d += rows_b + items_b;
+        i0 = i1;
+    }
+    NA_CUDA(cudaEventRecord(h->ev1, st));
+    return collect(h, b, rows, nh, found, res);
 }
 
 int run(hss_t* h, uint64_t first, uint64_t last, hss_counts* out, hss_hit* hits, uint32_t hit_cap,
@@ -256,36 +346,43 @@ int run(hss_t* h, uint64_t first, uint64_t last, hss_counts* out, hss_hit* hits,
     // work stack: whole rows, last row at the bottom
     uint32_t top = 0;
     for (uint32_t r = rows; r-- > 0;)
-        g_stack[top++] = Piece{r, (uint32_t)(first + r), (uint32_t)(h->limit + 1)};
+        g_stack[top++] = Piece{r, (uint32_t)(first + r), (uint32_t)(h->limit + 1), !h->plan};
     uint32_t max_group = kNaRows, nh = 0;
     uint64_t found = 0, h2d = rows * sizeof(RowInfo), d2h = 0;
     double ms = 0;
     uint32_t launches = 0;
     while (top) {
-        // a piece whose shared-prime pairs alone exceed the queue is halved
+        // a piece of products whose shared-prime pairs alone exceed the queue is halved
         const Piece& t = g_stack[top - 1];
-        if (shared_bound(h, g_host_rows[t.r].l, t.m0, t.m1) > kNaMerged) {
+        if (t.products && shared_bound(h, g_host_rows[t.r].l, t.m0, t.m1) > kNaMerged) {
             if (top + 1 > kNaPieces || t.m1 - t.m0 < 2 * kNaMinSpan)
                 return fail(h, HSS_ERR_OVERFLOW, "hss_search_noalloc: work stack full");
             const Piece p = t;
             const uint32_t mid = p.m0 + (p.m1 - p.m0) / 2;
-            g_stack[top - 1] = Piece{p.r, mid, p.m1};
-            g_stack[top++] = Piece{p.r, p.m0, mid};
+            g_stack[top - 1] = Piece{p.r, mid, p.m1, p.products};
+            g_stack[top++] = Piece{p.r, p.m0, mid, p.products};
             continue;
         }
-        // the group: pieces from the top while their shared-prime pairs fit
+        // the group: pieces of one kind from the top; of products while their
+        // shared-prime pairs fit
         uint32_t lo = top;
         uint64_t bound = 0;
         while (lo > 0 && top - lo < max_group) {
             const Piece& q = g_stack[lo - 1];
-            const uint64_t b = shared_bound(h, g_host_rows[q.r].l, q.m0, q.m1);
+            if (q.products != t.products) break;
+            const uint64_t b = !q.products ? 0 : shared_bound(h, g_host_rows[q.r].l, q.m0, q.m1);
             if (b > kNaMerged || bound + b > kNaMerged) break;
             bound += b;
             --lo;
         }
         GroupResult res{};
-        const int s = run_group(h, base, rows, lo, top, alpha_cap, &nh, &found, &res);
-        if (s == HSS_ERR_OVERFLOW) {
+        const int s = t.products ? run_group(h, base, rows, lo, top, alpha_cap, &nh, &found, &res)
+                                 : run_arc_group(h, base, rows, lo, top, &nh, &found, &res);
+        if (s == kNoRoom && top - lo == 1) {
+            g_stack[lo].products = true;
+            continue;
+        }
+        if (s == HSS_ERR_OVERFLOW || s == kNoRoom) {
             // run again smaller: half the pieces, or a lone piece halved
             if (top - lo > 1) {
                 max_group = (top - lo) / 2;
@@ -295,8 +392,8 @@ int run(hss_t* h, uint64_t first, uint64_t last, hss_counts* out, hss_hit* hits,
             if (top + 1 > kNaPieces || p.m1 - p.m0 < 2 * kNaMinSpan)
                 return fail(h, HSS_ERR_OVERFLOW, "hss_search_noalloc: a scratch queue overflowed");
             const uint32_t mid = p.m0 + (p.m1 - p.m0) / 2;
-            g_stack[lo] = Piece{p.r, mid, p.m1};
-            g_stack[top++] = Piece{p.r, p.m0, mid};
+            g_stack[lo] = Piece{p.r, mid, p.m1, p.products};
+            g_stack[top++] = Piece{p.r, p.m0, mid, p.products};
             continue;
         }
         if (s) return s;

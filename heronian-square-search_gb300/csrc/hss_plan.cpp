@@ -32,7 +32,7 @@ void ArcPlanner::clear() {
     rows.clear();
     rest.clear();
     items.clear();
-    keys.clear();
+    keys_.clear();
     entries = rest_pairs = 0;
 }
 
@@ -102,31 +102,47 @@ void ArcPlanner::add(const RowInfo& R, uint32_t row, uint64_t limit, uint32_t ma
             a.c3[f] = field_scale(f) * (p2m * p2m % M);
         }
         entries += a.na;
-        keys.push_back((uint64_t)s.p << 3 | ((l_class & 3) ? 4u : 0u) | (R.l3 ? 2u : 0u) | (R.l5 ? 1u : 0u));
+        keys_.push_back((uint64_t)s.p << 3 | ((l_class & 3) ? 4u : 0u) | (R.l3 ? 2u : 0u) | (R.l5 ? 1u : 0u));
         rows.push_back(a);
     }
 }
 
-void ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target) {
-    items.clear();
-    if (rows.empty()) return;
-    // rows by (P, parity, divisibility by 3 and 5), those of many values first
-    struct Order {
-        uint64_t key, rest;  // rest: values descending, then the order of addition
-    };
-    std::vector<Order> order(rows.size());
-    for (size_t i = 0; i < rows.size(); ++i) order[i] = Order{keys[i], (uint64_t)(UINT32_MAX - rows[i].na) << 32 | i};
-    std::sort(order.begin(), order.end(),
+// Rows by (P, parity, divisibility by 3 and 5), those of many values first.
+void ArcPlanner::sort() {
+    const size_t n = rows.size();
+    order_.resize(n);
+    sorted_.resize(n);
+    for (size_t i = 0; i < n; ++i) order_[i] = Order{keys_[i], (uint64_t)(UINT32_MAX - rows[i].na) << 32 | i};
+    std::sort(order_.begin(), order_.end(),
               [](const Order& x, const Order& y) { return x.key != y.key ? x.key < y.key : x.rest < y.rest; });
-    std::vector<ArcRow> sorted(rows.size());
-    uint32_t ent = 0;
-    for (size_t i = 0; i < order.size(); ++i) {
-        sorted[i] = rows[(uint32_t)order[i].rest];
-        keys[i] = order[i].key;
-        sorted[i].ent = ent;
-        ent += sorted[i].na;
+    for (size_t i = 0; i < n; ++i) {
+        sorted_[i] = rows[(uint32_t)order_[i].rest];
+        keys_[i] = order_[i].key;
     }
-    rows.swap(sorted);
+    rows.swap(sorted_);
+}
+
+void ArcPlanner::take(const ArcPlanner& from, size_t i0, size_t i1) {
+    clear();
+    for (size_t i = i0; i < i1; ++i) {
+        rows.push_back(from.rows[i]);
+        keys_.push_back(from.keys_[i]);
+        entries += from.rows[i].na;
+    }
+}
+
+bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target) {
+    items.clear();
+    groups_.clear();
+    if (rows.over() || keys_.over() || rest.over()) return false;
+    if (rows.empty()) return true;
+    sort();
+    uint32_t ent = 0;
+    for (size_t i = 0; i < rows.size(); ++i) {
+        rows[i].ent = ent;
+        ent += rows[i].na;
+    }
+    const Store<uint64_t>& keys = keys_;
     // the blocks of a type whose roots meet [lo, hi]
     auto range_of = [&](uint32_t t, uint32_t lo, uint32_t hi, uint32_t* b0, uint32_t* b1) {
         const uint32_t end = plan.type_first[t + 1];
@@ -142,11 +158,6 @@ void ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
         return !((key & 4u) && t >= 4) && !((key & 2u) && (t & 2u)) && !((key & 1u) && (t & 1u));
     };
     auto cost = [](const ArcRow& r) { return (uint64_t)r.na + 16; };
-    struct Group {
-        size_t g0, g1;
-        uint32_t b0[kTypes], b1[kTypes];  // its blocks of every type
-    };
-    std::vector<Group> groups;
     uint64_t total = 0;
     for (size_t g0 = 0; g0 < rows.size();) {
         size_t g1 = g0;
@@ -166,14 +177,14 @@ void ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
             range_of(t, lo, hi, &g.b0[t], &g.b1[t]);
             total += w * (g.b1[t] - g.b0[t]);
         }
-        groups.push_back(g);
+        groups_.push_back(g);
         g0 = g1;
     }
     // item size: the caller's, or about twelve items per resident CTA
     const uint64_t target = std::max<uint64_t>(16, item_target ? item_target : total / ((uint64_t)ctas * 12));
-    std::vector<ArcItem> cut;  // the group's chunks of rows, without a block
-    std::vector<uint32_t> cut_lo;
-    for (const Group& g : groups) {
+    Store<ArcItem>& cut = cut_;
+    Store<uint32_t>& cut_lo = cut_lo_;
+    for (const Group& g : groups_) {
         cut.clear();
         cut_lo.clear();
         for (size_t i = g.g0; i < g.g1;) {
@@ -201,12 +212,15 @@ void ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
             for (uint32_t b = g.b0[t]; b < g.b1[t]; ++b)
                 for (size_t c = 0; c < cut.size(); ++c) {
                     if (cut_lo[c] > plan.blocks[b].m_hi) continue;
-                    items.push_back(cut[c]);
-                    items.back().block = b;
-                    items.back().base = plan.blocks[b].base;
-                    items.back().n = (uint16_t)plan.blocks[b].n;
+                    ArcItem item = cut[c];
+                    item.block = b;
+                    item.base = plan.blocks[b].base;
+                    item.n = (uint16_t)plan.blocks[b].n;
+                    items.push_back(item);
                 }
+        if (items.over()) return false;
     }
+    return true;
 }
 
 }  // namespace hss

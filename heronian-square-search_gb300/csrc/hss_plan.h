@@ -2,12 +2,70 @@
 #pragma once
 #include <stdint.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "hss_blocks.h"
 #include "hss_kernels.h"
 
 namespace hss {
+
+// The planner's arrays: grown as needed, or over memory that is given once and
+// never exceeded (over() then tells that an entry found no room).
+template <class T>
+class Store {
+  public:
+    void fix(T* p, size_t cap) {
+        p_ = p;
+        cap_ = cap;
+        fixed_ = true;
+    }
+    void push_back(const T& x) {
+        if (n_ == cap_ && !grow(n_ + 1)) return;
+        p_[n_++] = x;
+    }
+    void resize(size_t n) {
+        if (n > cap_ && !grow(n)) n = cap_;
+        n_ = n;
+    }
+    void clear() {
+        n_ = 0;
+        over_ = false;
+    }
+    void swap(Store& o) {
+        own_.swap(o.own_);
+        std::swap(p_, o.p_);
+        std::swap(n_, o.n_);
+        std::swap(cap_, o.cap_);
+        std::swap(fixed_, o.fixed_);
+        std::swap(over_, o.over_);
+    }
+    size_t size() const { return n_; }
+    bool empty() const { return n_ == 0; }
+    bool over() const { return over_; }
+    T* data() { return p_; }
+    T* begin() { return p_; }
+    T* end() { return p_ + n_; }
+    T& back() { return p_[n_ - 1]; }
+    T& operator[](size_t i) { return p_[i]; }
+    const T& operator[](size_t i) const { return p_[i]; }
+
+  private:
+    bool grow(size_t n) {
+        if (fixed_) {
+            over_ = true;
+            return false;
+        }
+        own_.resize(std::max(n, 2 * cap_));
+        p_ = own_.data();
+        cap_ = own_.size();
+        return true;
+    }
+    std::vector<T> own_;
+    T* p_ = nullptr;
+    size_t n_ = 0, cap_ = 0;
+    bool fixed_ = false, over_ = false;
+};
 
 // Roots m' below which the pairs of a common part P are handed to the
 // shared-prime kernels, for a call of `rows` roots.
@@ -25,16 +83,55 @@ class ArcPlanner {
     void add(const RowInfo& R, uint32_t row, uint64_t limit, uint32_t max_exponent, uint64_t m0, uint64_t m1,
              uint64_t least);
     // Orders the rows, assigns their values' entries and builds the items.
-    void finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target);
+    // False when an array over given memory had no room.
+    bool finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target);
+    // Orders the rows as finish does, and takes rows [i0, i1) of another planner.
+    void sort();
+    void take(const ArcPlanner& from, size_t i0, size_t i1);
 
-    std::vector<ArcRow> rows;
-    std::vector<ArcRest> rest;
-    std::vector<ArcItem> items;
+    // Arrays over given memory, for callers that may not allocate.
+    struct Order {
+        uint64_t key, rest;  // rest: values descending, then the order of addition
+    };
+    struct Group {
+        size_t g0, g1;
+        uint32_t b0[kTypes], b1[kTypes];  // its blocks of every type
+    };
+    template <size_t ROWS, size_t ITEMS>
+    struct Arena {
+        ArcRow rows[ROWS], sorted[ROWS];
+        ArcItem items[ITEMS], cut[ROWS];
+        uint64_t keys[ROWS];
+        uint32_t cut_lo[ROWS];
+        Order order[ROWS];
+        Group groups[ROWS];
+    };
+    template <size_t ROWS, size_t ITEMS>
+    void use(Arena<ROWS, ITEMS>& a) {
+        rows.fix(a.rows, ROWS);
+        sorted_.fix(a.sorted, ROWS);
+        items.fix(a.items, ITEMS);
+        cut_.fix(a.cut, ROWS);
+        keys_.fix(a.keys, ROWS);
+        cut_lo_.fix(a.cut_lo, ROWS);
+        order_.fix(a.order, ROWS);
+        groups_.fix(a.groups, ROWS);
+        rest.fix(nullptr, 0);
+    }
+
+    Store<ArcRow> rows;
+    Store<ArcRest> rest;
+    Store<ArcItem> items;
     uint64_t entries = 0;     // values of all rows
     uint64_t rest_pairs = 0;  // pairs of the rest list at most
 
   private:
-    std::vector<uint64_t> keys;  // sort key of rows[i]
+    Store<uint64_t> keys_;  // sort key of rows[i]
+    Store<ArcRow> sorted_;
+    Store<Order> order_;
+    Store<Group> groups_;
+    Store<ArcItem> cut_;  // the group's chunks of rows, without a block
+    Store<uint32_t> cut_lo_;
 };
 
 }  // namespace hss

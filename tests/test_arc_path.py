@@ -2,7 +2,8 @@
 which evaluates every Gaussian product: the smallest arc limit, the one below
 it, the last row, low rows (shared primes and powers with most roots), heavy
 rows of each parity, a limit with ragged last blocks, a call long enough to be
-planned in two pieces, both CTA sizes and a captured graph."""
+planned in two pieces, both CTA sizes and a captured graph.  And the no-alloc
+form by arcs against the batched one, on two calls in a row."""
 import pytest
 
 import hss
@@ -31,3 +32,20 @@ def test_batched_equals_plain(limit, first, last, opts):
         assert {k: got.counts[k] for k in FIELDS} == {k: plain.counts[k] for k in FIELDS}
         assert got.row_candidates == plain.row_candidates
         assert got.hits == plain.hits
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit,first,last", [
+    (11_999, 11_990, 11_999),
+    (12_000, 1, 64),
+    (12_000, 11_937, 12_000),
+    (300_017, 160_222, 160_228),
+    (5_000_000, 1_185_665, 1_185_665),
+])
+def test_noalloc_equals_batched(limit, first, last):
+    with hss.Search(limit) as s:
+        want = s.search(first, last)
+        for _ in range(2):
+            got = s.search_noalloc(first, last)
+            assert {k: got.counts[k] for k in FIELDS} == {k: want.counts[k] for k in FIELDS}
+            assert got.hits == want.hits
