@@ -38,7 +38,9 @@ constexpr uint32_t kDefaultItemTarget = 1u << 23;
 constexpr uint32_t kTileCap = 16384;           // largest m-range of one item
 constexpr uint32_t kTileMin = 32;
 constexpr uint32_t kBucketShift = 10;          // item ordering granularity in m
-constexpr uint64_t kArcLimit = 12000;          // the arc path from this limit on (see run_batched)
+constexpr uint64_t kArcLeast = 1000;            // handles from this limit on have the arc layout
+constexpr uint64_t kArcLimit = 10000;          // and long calls use it from this one on (see run_batched)
+constexpr size_t kArcRows = 64;
 constexpr uint64_t kMergedCap = 96ull << 20;   // shared-prime queue entries
 constexpr uint32_t kDescChunk = 1u << 24;       // shared-prime pairs set up per chunk (192 bytes each: 3 GB)
 // With the arc layout only the rest list's few pairs come by the shared-prime
@@ -597,12 +599,15 @@ constexpr uint64_t kGroupValues = 8ull << 20;
 constexpr size_t kGroupRows = 1u << 20;
 constexpr size_t kLongCall = 2048;
 
-// Below kArcLimit the product kernel stays the faster path: class lists are too
-// short there for runs to pay (roots 80..4979 at LIMIT 5000: 3.3 ms by
-// products, 4.3 ms by arcs; 1..3000 at 3000: 1.5 and 2.3; 8000..9999 at 10^4: 1.5
-// and 1.3; 5000..7000 at 20,000: 10.6 and 6.1).
+// Long calls below kArcLimit go by products: class lists are too short there
+// for runs to pay (roots 80..4979 at LIMIT 5000: 3.3 ms by products, 4.1 ms by
+// arcs; 100..7000 at 8000: 7.4 and 8.3; 4000..4100 at 5000: 0.39 and 0.46; but
+// 3000..5000 at 11,000: 4.5 and 3.8).  Calls of at most kArcRows roots spend their
+// time on launches and waits, of which the arc path has fewer (four roots at
+// 8000: 0.36 ms by products, 0.13 by arcs; one at 2000 or 5000: 0.29 and 0.25, 0.39 and
+// 0.18).
 int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
-    if (!h->plan) return run_products(h, rows);
+    if (!h->plan || (h->limit < kArcLimit && rows.size() > kArcRows)) return run_products(h, rows);
     h->planner.clear();
     size_t start = 0;
     if (int s = ensure_row_info(h, rows.size())) return s;
@@ -740,7 +745,7 @@ void copy_hits(const std::vector<DevHit>& in, hss_hit* out, uint32_t cap) {
 
 // The arc layout of the handle's cache (h->dev, h->records), enqueued on the stream.
 int open_arc_layout(hss_t* h) {
-    if (h->limit < kArcLimit) return HSS_OK;
+    if (h->limit < kArcLeast) return HSS_OK;
     auto plan = std::make_shared<ArcPlan>();
     ArcBuild b;
     std::string err;

@@ -55,6 +55,7 @@ constexpr uint32_t kArcQueue = 96;           // events per warp: under 32 kept, 
 // marked entries with ranks, and the event queue.
 constexpr uint32_t kArcCap = kBlockEntries + 32;  // the filter's last round reads past a run's end
 constexpr uint32_t kArcWords = kArcCap / 32;
+static_assert(kIndexWords % 4 == 0 && sizeof(ArcBlock) % 16 == 0, "prefetched in 16-byte pieces");
 static_assert(kArcCap % 32 == 0 && kArcCap < 65536, "whole words, 16-bit positions");
 // The filter's 12 constants of one gamma: per field the multipliers of the
 // packed word, of it >> 10 and of it >> 20, and the row's term.  With
@@ -219,12 +220,8 @@ struct ArcCounts {
 };
 
 __device__ __forceinline__ bool arc_prepare(const DeviceCache& cache, const ArcBuffers& buf, const ArcBlock& B,
-                                            const uint32_t* s_ang, uint32_t v, ArcSlot& S, uint32_t* bits,
+                                            const uint32_t* s_ang, ArcSlot& S, uint32_t* bits,
                                             uint16_t* rank, uint4* range, uint32_t lane, ArcCounts& out) {
-    __syncwarp();
-    if (lane < sizeof(ArcRow) / 4)
-        reinterpret_cast<uint32_t*>(&S.row)[lane] = reinterpret_cast<const uint32_t*>(buf.arc_rows + v)[lane];
-    __syncwarp();
     const ArcRow& row = S.row;
     const RowInfo& R = buf.row_info[row.row];
     const uint32_t lo = max(B.m_lo, row.m_lo), hi = min(B.m_hi, row.m_hi);
@@ -611,9 +608,6 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
             for (uint32_t k = tid; k < kIndexWords; k += NT)
                 M.index[k] = cache.arc_index[(size_t)w.block * kIndexWords + k];
         }
-        // class rules of the item's rows (one parity, one divisibility by 3
-        // and 5) against the block's type
-        const uint32_t lc = buf.arc_rows[w.v0].l_class;
         // the next item, and its block towards L2 while this one runs
         if (tid == NT - 1) {
             const uint32_t ahead = atomicAdd(buf.next_item, 1u);
@@ -622,9 +616,13 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                 const ArcItem x = items[ahead];
                 const uint32_t quads = (x.n + 3u) / 4;
                 if (x.block != w.block && quads) {
+                    // (whole quads: 16-byte sizes, from 16-byte boundaries)
 #pragma unroll
                     for (uint32_t f = 0; f < kFields; ++f) arc_prefetch(cache.arc_w[f] + x.base, quads);
                     arc_prefetch(cache.arc_ang + x.base, quads);
+                    arc_prefetch(reinterpret_cast<const uint32_t*>(cache.arc_part + x.base), (x.n + 15u) / 16);
+                    arc_prefetch(cache.arc_index + (size_t)x.block * kIndexWords, kIndexWords / 4);
+                    arc_prefetch(reinterpret_cast<const uint32_t*>(cache.blocks + x.block), sizeof(ArcBlock) / 16);
                 }
             }
         }
@@ -632,11 +630,6 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
         __syncthreads();
         const ArcBlock& B = S.block;
         const uint32_t type = B.type, block0 = B.base;
-        const bool odd = type < 4 && (lc & 3u) == 0;
-        const uint32_t defined = (type < 4 ? 4u : 0u) | ((type & 2u) ? 0u : 2u) | ((type & 1u) ? 0u : 1u);
-        const uint32_t match = defined & (((lc & 4u) ? 0u : 2u) | ((lc & 8u) ? 0u : 1u));
-        const uint32_t open = defined & ~match;
-        const uint32_t lf = __popc(open), lu = odd ? 1u : 2u, lt = lf + 2u + lu;
         // warps take rows (or parts of rows) on their own
         const uint32_t shared = w.split * w.parts, units = (shared + w.nv - w.split) * w.share;
         for (;;) {
@@ -646,16 +639,33 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
             if (unit >= units) break;
             // of the runs of a group, this warp's: lanes = turn mod share
             const uint32_t turn = unit % w.share;
-            const uint32_t mask_mine = (w.share == 1 ? kFull : w.share == 2 ? 0x55555555u : w.share == 4 ? 0x11111111u : 0x01010101u) << turn;
+            const uint32_t mask_mine = kFull / ((w.share < 32 ? 1u << w.share : 0u) - 1u) << turn;  // share a power of two
             unit /= w.share;
             const bool whole = unit >= shared;
             const uint32_t parts = whole ? 1u : w.parts, part = whole ? 0u : unit % parts;
             const uint32_t v = w.v0 + (whole ? unit - shared + w.split : unit / parts);
+            __syncwarp();
+            if (lane < sizeof(ArcRow) / 4)
+                reinterpret_cast<uint32_t*>(&T.row)[lane] = reinterpret_cast<const uint32_t*>(buf.arc_rows + v)[lane];
+            __syncwarp();
+            // class rules of the row against the block's type; l and m' have no
+            // common factor 2, 3 or 5
+            const uint32_t lc = T.row.l_class;
+            if (((lc & 3u) && type >= 4) || ((lc & 4u) && (type & 2u)) || ((lc & 8u) && (type & 1u))) continue;
+            {
+                const uint32_t defined = (type < 4 ? 4u : 0u) | ((type & 2u) ? 0u : 2u) | ((type & 1u) ? 0u : 1u);
+                const uint32_t match = defined & (((lc & 4u) ? 0u : 2u) | ((lc & 8u) ? 0u : 1u));
+                const bool odd = type < 4 && (lc & 3u) == 0;
+                const bool always = (lc & 3u) == 2u || type >= 8u;  // even pairs: z = 1 mod 16 whatever D
+                const uint32_t lu = odd ? 1u : 2u, lt = __popc(defined & ~match) + 2u + lu;
+                const uint32_t runs1 = T.row.na << lt, runs2 = (T.row.na - 1) << lu;
+                if (32 * part >= runs1 + runs2) continue;  // no runs left for this part
+                // (kept in shared memory, away from the filter's registers)
+                if (lane == 0) T.row.rules = match | (defined & ~match) << 3 | (odd ? 64u : 0u) | (always ? 128u : 0u) | lt << 8;
+            }
             ArcCounts counts;
-            if (!arc_prepare(cache, buf, B, s_ang, v, T, W.bits, W.rank, W.range, lane, counts)) continue;
+            if (!arc_prepare(cache, buf, B, s_ang, T, W.bits, W.rank, W.range, lane, counts)) continue;
             const bool excl = counts.excl;
-            const uint32_t na = T.row.na, ent0 = T.row.ent, runs1 = na << lt, runs2 = (na - 1) << lu;
-            const bool always = (T.row.l_class & 3u) == 2u || type >= 8u;  // even pairs: z = 1 mod 16 whatever D
             const uint32_t k0[kFields] = {T.row.c0[0], T.row.c0[1], T.row.c0[2]};
             auto marked = [&](uint32_t i) { return ((W.bits[i >> 5] >> (i & 31u)) & 1u) != 0; };
             if (lane == 0) W.cand = W.r16 = 0;
@@ -669,8 +679,13 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                 }
                 open_n += __popc(mask);
             };
-            for (uint32_t t0 = 32 * part; t0 < runs1 + runs2; t0 += 32 * parts) {
+            auto runs_of_row = [&] { return (T.row.na << (T.row.rules >> 8)) + ((T.row.na - 1) << ((T.row.rules & 64u) ? 1 : 2)); };
+            for (uint32_t t0 = 32 * part; t0 < runs_of_row(); t0 += 32 * parts) {
                 uint32_t t = t0 + lane;
+                const uint32_t rules = T.row.rules, na = T.row.na, ent0 = T.row.ent;
+                const uint32_t match = rules & 7u, open = (rules >> 3) & 7u, lt = rules >> 8;
+                const bool odd = (rules & 64u) != 0, always = (rules & 128u) != 0;
+                const uint32_t lu = odd ? 1u : 2u, runs1 = na << lt;
                 // the lane's run: possible [p0, p1), certain [c0, c1)
                 uint32_t p0 = 0, p1 = 0, c0 = 0, c1 = 0, id = 0, ang0 = 0;
                 bool keep = false;  // z = 0, 1 mod 16
@@ -678,7 +693,7 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                     uint32_t sub = 0;
                     {
                         uint32_t bitsel = open;
-                        for (uint32_t f = 0; f < lf; ++f) {
+                        while (bitsel) {
                             const uint32_t b = bitsel & (0u - bitsel);
                             if (t & 1u) sub |= b;
                             t >>= 1;
@@ -715,7 +730,7 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                             }
                         }
                     }
-                } else if (t - runs1 < runs2) {
+                } else if (t < runs_of_row()) {
                     t -= runs1;
                     const uint32_t u = odd ? (t & 1u) * 2u : t & 3u, k = t >> lu;
                     const uint32_t cls = buf.arc_values[ent0 + k].cls ^ ((u & 1u) ? 3u : 0u) ^ ((u & 2u) ? 4u : 0u);
@@ -781,7 +796,7 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                     in = x >= r.x && x <= r.z;
                     doubtful = !in && x >= r.y && x <= r.w;
                 };
-                const bool final = t0 + 32 * parts >= runs1 + runs2;  // the unit's last runs
+                const bool final = t0 + 32 * parts >= runs_of_row();  // the unit's last runs
                 uint32_t at = 0, end = 0, tag = 0, ang_run = 0, base = 0;
                 bool check = false;
                 ArcFilter c{};
@@ -918,7 +933,7 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                     cand += counts.cc;
                     r16 += counts.cc;
                     const unsigned long long products =
-                        (2ull * na - 1) * counts.records - (unsigned long long)(na - 1) * counts.processed;
+                        (2ull * T.row.na - 1) * counts.records - (unsigned long long)(T.row.na - 1) * counts.processed;
                     if (counts.processed) {
                         atomicAdd(&rc->processed, (unsigned long long)counts.processed);
                         atomicAdd(&rc->products, products);

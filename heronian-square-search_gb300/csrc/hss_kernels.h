@@ -72,12 +72,12 @@ struct ArcRow {
     float zscale;              // 2 l^2 P^2: |gamma beta| / m'^2
     float lw_hi, lw_lo;        // l^4 - N^4 in two floats
     uint32_t l_class;          // 0 odd, 1 = 2 mod 4, 2 = 0 mod 4; + 4 if 3 | l; + 8 if 5 | l
-    uint32_t pad;
+    uint32_t rules;            // in a warp's copy: the class rules against its block's type
 };
 static_assert(sizeof(ArcRow) == 80, "arc row is 80 bytes");
 
-// One unit of arc work: rows v0 .. v0 + nv - 1 (one l_class parity and the
-// same divisibility by 3 and 5) against one block.  Warps take whole rows,
+// One unit of arc work: rows v0 .. v0 + nv - 1 against one block (those whose
+// class or range leaves the block out are passed over).  Warps take whole rows,
 // except for the first `split` rows (those of many values), whose groups of
 // 32 runs are shared by `parts` warps each; where an item has too few rows for
 // its warps even so, `share` warps take every share-th run of a group.

@@ -8,6 +8,9 @@
 namespace hss {
 namespace {
 
+constexpr size_t kMergedRows = 64;  // most rows of an item of several groups
+constexpr uint64_t kMergedCost = 1000;  // and their cost at most (400 and 4,000: within 2 %)
+
 using u128 = unsigned __int128;
 using i128 = __int128;
 
@@ -172,6 +175,7 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
         Group g{};
         g.g0 = g0;
         g.g1 = g1;
+        g.cost = w;
         for (uint32_t t = 0; t < kTypes; ++t) {
             if (!type_allowed(keys[g0], t)) continue;
             range_of(t, lo, hi, &g.b0[t], &g.b1[t]);
@@ -182,9 +186,70 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
     }
     // item size: the caller's, or about twelve items per resident CTA
     const uint64_t target = std::max<uint64_t>(16, item_target ? item_target : total / ((uint64_t)ctas * 12));
+    const uint64_t merged = std::min<uint64_t>(std::max<uint64_t>(target, 400), kMergedCost);
     Store<ArcItem>& cut = cut_;
     Store<uint32_t>& cut_lo = cut_lo_;
-    for (const Group& g : groups_) {
+    auto emit = [&](ArcItem item, uint32_t b) {
+        item.block = b;
+        item.base = plan.blocks[b].base;
+        item.n = (uint16_t)plan.blocks[b].n;
+        items.push_back(item);
+    };
+    for (size_t x = 0; x < groups_.size();) {
+        // Groups that fit one item together share it: a block is loaded and waited
+        // for once for all of them.  With an item per group, three rows at LIMIT 10^7
+        // spent 43 to 79 % of their time on loads and barriers: 4.5 ms and 2.4 ms so
+        // (l = 331,000), 10.8 and 8.1 ms (l = 160,000); 8 rows at 7.5 10^6 4.8 and 2.9 ms,
+        // 37 near the limit 1.75 and 1.5 ms.  Groups above kMergedCost hold enough
+        // work per block by themselves.
+        size_t y = x + 1;
+        uint64_t w = groups_[x].cost;
+        while (y < groups_.size() && w + groups_[y].cost <= merged && groups_[y].g1 - groups_[x].g0 <= kMergedRows)
+            w += groups_[y++].cost;
+        if (y - x > 1) {
+            for (uint32_t t = 0; t < kTypes; ++t) {
+                // between the ends of the groups' ranges the groups that meet a block stay the same
+                uint32_t edge[2 * kMergedRows];
+                size_t n = 0;
+                for (size_t i = x; i < y; ++i) {
+                    if (groups_[i].b0[t] == groups_[i].b1[t]) continue;
+                    edge[n++] = groups_[i].b0[t];
+                    edge[n++] = groups_[i].b1[t];
+                }
+                std::sort(edge, edge + n);
+                for (size_t k = 0; k + 1 < n; ++k) {
+                    if (edge[k] == edge[k + 1]) continue;
+                    size_t first = y, last = x;
+                    uint64_t units = 0, sum = 0;
+                    uint32_t most = 1;
+                    for (size_t i = x; i < y; ++i) {
+                        if (groups_[i].b0[t] > edge[k] || groups_[i].b1[t] <= edge[k]) continue;
+                        first = std::min(first, i);
+                        last = i;
+                    }
+                    if (first == y) continue;
+                    const size_t v0 = groups_[first].g0, nv = groups_[last].g1 - v0;
+                    for (size_t i = 0; i < nv; ++i) {
+                        most = std::max(most, rows[v0 + i].na);
+                        sum += cost(rows[v0 + i]);
+                    }
+                    // rows in up to `parts` parts (a part holds at least 32 runs; what
+                    // is past a row's last run is passed over), so that there is a
+                    // unit per warp and none holds more than a forty-eighth
+                    const uint64_t want = std::max<uint64_t>(24 / nv, ((most + 16) * 48 + sum - 1) / sum);
+                    const uint32_t parts = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({want, 24, (most + 1) / 2}));
+                    for (size_t i = 0; i < nv; ++i) units += std::min(parts, (rows[v0 + i].na + 1) / 2);
+                    uint32_t share = 1;
+                    for (; units < 16 && share < 8; units *= 2) share *= 2;
+                    const ArcItem item{0, 0, (uint32_t)v0, (uint16_t)nv, (uint16_t)nv, (uint16_t)parts, 0, share};
+                    for (uint32_t b = edge[k]; b < edge[k + 1]; ++b) emit(item, b);
+                }
+            }
+            x = y;
+            if (items.over()) return false;
+            continue;
+        }
+        const Group& g = groups_[x++];
         cut.clear();
         cut_lo.clear();
         for (size_t i = g.g0; i < g.g1;) {
@@ -201,23 +266,18 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
             // (a part holds at least a few groups of 32 runs)
             const uint64_t parts =
                 split ? std::max<uint64_t>(1, std::min({(uint64_t)24, (cost(rows[i]) * 48 + w - 1) / w, (uint64_t)rows[i].na / 2})) : 1;
-            cut.push_back(ArcItem{0, 0, (uint32_t)i, (uint16_t)(e - i), (uint16_t)split, (uint16_t)parts, 0, 1});
+            ArcItem item{0, 0, (uint32_t)i, (uint16_t)(e - i), (uint16_t)split, (uint16_t)parts, 0, 1};
             // fewer units than warps: the runs of a group are shared too
             uint64_t units = split * parts + (e - i - split);
-            for (; units < 16 && cut.back().share < 8; units *= 2) cut.back().share *= 2;
+            for (; units < 16 && item.share < 8; units *= 2) item.share *= 2;
+            cut.push_back(item);
             cut_lo.push_back(lo);
             i = e;
         }
         for (uint32_t t = 0; t < kTypes; ++t)
             for (uint32_t b = g.b0[t]; b < g.b1[t]; ++b)
-                for (size_t c = 0; c < cut.size(); ++c) {
-                    if (cut_lo[c] > plan.blocks[b].m_hi) continue;
-                    ArcItem item = cut[c];
-                    item.block = b;
-                    item.base = plan.blocks[b].base;
-                    item.n = (uint16_t)plan.blocks[b].n;
-                    items.push_back(item);
-                }
+                for (size_t c = 0; c < cut.size(); ++c)
+                    if (cut_lo[c] <= plan.blocks[b].m_hi) emit(cut[c], b);
         if (items.over()) return false;
     }
     return true;

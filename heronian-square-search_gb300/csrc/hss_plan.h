@@ -94,7 +94,8 @@ class ArcPlanner {
         uint64_t key, rest;  // rest: values descending, then the order of addition
     };
     struct Group {
-        size_t g0, g1;
+        size_t g0, g1;            // rows of one key
+        uint64_t cost;
         uint32_t b0[kTypes], b1[kTypes];  // its blocks of every type
     };
     template <size_t ROWS, size_t ITEMS>

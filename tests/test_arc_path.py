@@ -1,6 +1,7 @@
-"""The batched form by arcs (limits from 12,000 on) against the plain form,
-which evaluates every Gaussian product: the smallest arc limit, the one below
-it, the last row, low rows (shared primes and powers with most roots), heavy
+"""The batched form by arcs against the plain form, which evaluates every
+Gaussian product: the smallest limit with the arc layout and the one below it,
+calls of 64 and 65 rows below the limit from which long calls go by arcs, that
+limit and the one below it, the last row, low rows (shared primes and powers with most roots), heavy
 rows of each parity, a limit with ragged last blocks, a call long enough to be
 planned in two pieces, both CTA sizes and a captured graph.  And the no-alloc
 form by arcs against the batched one, on two calls in a row."""
@@ -13,7 +14,13 @@ FIELDS = ("pairs", "processed", "products", "candidates", "r16", "merged", "merg
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("limit,first,last,opts", [
-    (11_999, 11_400, 11_999, {}),
+    (999, 1, 64, {}),
+    (1_000, 1, 64, {}),
+    (5_000, 4_937, 5_000, {}),
+    (5_000, 1, 65, {}),
+    (9_999, 1_100, 1_163, {}),
+    (9_999, 9_399, 9_999, {}),
+    (10_000, 9_400, 10_000, {}),
     (12_000, 1, 70, {}),
     (12_000, 11_400, 12_000, {}),
     (12_000, 5_000, 7_100, {}),
@@ -36,7 +43,8 @@ def test_batched_equals_plain(limit, first, last, opts):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("limit,first,last", [
-    (11_999, 11_990, 11_999),
+    (999, 100, 163),
+    (1_000, 937, 1_000),
     (12_000, 1, 64),
     (12_000, 11_937, 12_000),
     (300_017, 160_222, 160_228),
