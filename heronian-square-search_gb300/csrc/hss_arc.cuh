@@ -219,7 +219,7 @@ struct ArcCounts {
     bool excl;
 };
 
-__device__ __forceinline__ bool arc_prepare(const DeviceCache& cache, const ArcBuffers& buf, const ArcBlock& B,
+__device__ __forceinline__ bool arc_prepare(const ArcCache& cache, const ArcBuffers& buf, const ArcBlock& B, uint32_t block,
                                             const uint32_t* s_ang, ArcSlot& S, uint32_t* bits,
                                             uint16_t* rank, uint4* range, uint32_t lane, ArcCounts& out) {
     const ArcRow& row = S.row;
@@ -278,9 +278,17 @@ __device__ __forceinline__ bool arc_prepare(const DeviceCache& cache, const ArcB
         r0 = roots_upto(c_arc_types, B.type, (lo - 1) / p);
         multiples = roots_upto(c_arc_types, B.type, hi / p) - r0;
     }
+    // Small primes have their bit sets ready, so that most rows gather little or
+    // nothing: three rows at LIMIT 10^7 (l = 160,000) 8.1 ms without them and 5.1 ms
+    // with, 37 near the limit 1.5 and 1.35, 512 rows 125 and 121.
+    uint32_t small = __ballot_sync(kFull, multiples != 0 && p <= mask_prime(kMaskPrimes - 1));
+    const bool masks = small != 0;
+    uint32_t pick = 0, picked = 0;  // which of them, four bits each
+    for (; small; small &= small - 1) pick |= mask_of(__shfl_sync(kFull, p, __ffs(small) - 1)) << (4 * picked++);
+    if (p <= mask_prime(kMaskPrimes - 1)) multiples = 0;
     const uint32_t incl_p = arc_scan(multiples, lane), all = __shfl_sync(kFull, incl_p, 31);
     const uint32_t words = (B.n + 31) / 32;
-    const bool excl = trim || all != 0;
+    const bool excl = trim || masks || all != 0;
     uint32_t marked = 0, marked_roots = 0;
     if (excl) {
         if (trim) {
@@ -302,7 +310,15 @@ __device__ __forceinline__ bool arc_prepare(const DeviceCache& cache, const ArcB
             for (uint32_t i = lane; i < words; i += 32) bits[i] = 0;
         }
         __syncwarp();
-        // the multiples, 32 roots at a time; their records laid end to end
+        const uint32_t* mask = cache.arc_mask + (size_t)block * (kMaskPrimes * kMaskWords);
+        for (uint32_t k = 0; k < picked; ++k) {
+            const uint32_t* set = mask + ((pick >> (4 * k)) & 15u) * kMaskWords;
+#pragma unroll
+            for (uint32_t q = 0; q < kMaskWords / 32; ++q)
+                if (32 * q + lane < words) bits[32 * q + lane] |= set[32 * q + lane];
+        }
+        __syncwarp();
+        // multiples of the larger primes, 32 roots at a time; their records laid end to end
         for (uint32_t b0 = 0; b0 < all; b0 += 32) {
             const uint32_t own = arc_owner(incl_p, b0 + lane);
             const uint32_t q = __shfl_sync(kFull, p, own), k0 = __shfl_sync(kFull, r0, own);
@@ -387,7 +403,7 @@ __device__ __forceinline__ bool arc_prepare(const DeviceCache& cache, const ArcB
 // scans the candidate roots of all lanes together, and possible hits go to
 // the exact kernel.
 // Inlined at the kernel's two drains: no call in the kernel.
-__device__ __forceinline__ void arc_events(uint32_t at, uint32_t v, uint32_t ev, bool live, const DeviceCache& cache,
+__device__ __forceinline__ void arc_events(uint32_t at, uint32_t v, uint32_t ev, bool live, const ArcCache& cache,
                                            const ArcBuffers& buf) {
     const uint32_t lane = threadIdx.x & 31, var = ev & 7u, ent = ev >> 3;
     uint32_t nlo = 1, nhi = 0, zres = 0, j = 0, m1 = 0, row_id = 0, m = 0, l = 0;
@@ -519,7 +535,7 @@ __device__ __forceinline__ bool arc_piece(uint32_t start, uint32_t len, uint32_t
 }
 
 template <int NT>
-__global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ DeviceCache cache,
+__global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ ArcCache cache,
                                                        const ArcItem* __restrict__ items, uint32_t n_items,
                                                        const __grid_constant__ ArcBuffers buf) {
     constexpr uint32_t kWarps = NT / 32;
@@ -621,6 +637,7 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                     for (uint32_t f = 0; f < kFields; ++f) arc_prefetch(cache.arc_w[f] + x.base, quads);
                     arc_prefetch(cache.arc_ang + x.base, quads);
                     arc_prefetch(reinterpret_cast<const uint32_t*>(cache.arc_part + x.base), (x.n + 15u) / 16);
+                    arc_prefetch(cache.arc_mask + (size_t)x.block * (kMaskPrimes * kMaskWords), kMaskPrimes * kMaskWords / 4);
                     arc_prefetch(cache.arc_index + (size_t)x.block * kIndexWords, kIndexWords / 4);
                     arc_prefetch(reinterpret_cast<const uint32_t*>(cache.blocks + x.block), sizeof(ArcBlock) / 16);
                 }
@@ -664,7 +681,7 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ Devi
                 if (lane == 0) T.row.rules = match | (defined & ~match) << 3 | (odd ? 64u : 0u) | (always ? 128u : 0u) | lt << 8;
             }
             ArcCounts counts;
-            if (!arc_prepare(cache, buf, B, s_ang, T, W.bits, W.rank, W.range, lane, counts)) continue;
+            if (!arc_prepare(cache, buf, B, w.block, s_ang, T, W.bits, W.rank, W.range, lane, counts)) continue;
             const bool excl = counts.excl;
             const uint32_t k0[kFields] = {T.row.c0[0], T.row.c0[1], T.row.c0[2]};
             auto marked = [&](uint32_t i) { return ((W.bits[i >> 5] >> (i & 31u)) & 1u) != 0; };

@@ -140,7 +140,7 @@ inline size_t block_sort_smem(uint32_t cap) { return kHistWords * 4 + (size_t)ca
 __global__ void __launch_bounds__(kBlockThreads) block_sort_kernel(
     ArcBlock* blocks, uint32_t cap, const uint32_t* __restrict__ seg_off, const HotRec* __restrict__ hot,
     const ExactRec* __restrict__ exact, const uint32_t* __restrict__ owner, uint32_t* w0, uint32_t* w1, uint32_t* w2,
-    uint32_t* ang, uint8_t* part, uint32_t* src, uint32_t* root, float2* xy, uint32_t* index, uint16_t* pos) {
+    uint32_t* ang, uint8_t* part, uint32_t* src, uint32_t* root, float2* xy, uint32_t* index, uint32_t* mask, uint16_t* pos) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t* s_hist = reinterpret_cast<uint32_t*>(smem);
     uint32_t* s_key = s_hist + kHistWords;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kBlockThreads) block_sort_kernel(
     __syncthreads();
     // exclusive scan of the histogram
     constexpr uint32_t kEach = kHist / kBlockThreads;
-    static_assert(kHist % kBlockThreads == 0, "");
+    static_assert(kHist % kBlockThreads == 0 && kBlockEntries % kBlockThreads == 0, "whole rounds");
     uint32_t sum = 0;
     for (uint32_t i = 0; i < kEach; ++i) sum += s_hist[hist_at(tid * kEach + i)];
     uint32_t incl = sum;
@@ -273,6 +273,19 @@ __global__ void __launch_bounds__(kBlockThreads) block_sort_kernel(
         root[at] = m;
         xy[at] = make_float2(h.re, fabsf(h.im));
         pos[j] = (uint16_t)place;
+    }
+    __syncthreads();
+    // the small primes' bit sets, a word per warp at a time
+    uint32_t* sets = mask + (size_t)blockIdx.x * (kMaskPrimes * kMaskWords);
+    for (uint32_t i = tid; i < kBlockEntries; i += kBlockThreads) {
+        const uint32_t m = i < B.n ? root[B.base + i] : 1u;
+        uint32_t word = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kMaskPrimes; ++q) {
+            const uint32_t set = __ballot_sync(0xFFFFFFFFu, m % mask_prime(q) == 0);
+            if (lane == q) word = set;
+        }
+        if (lane < kMaskPrimes) sets[lane * kMaskWords + i / 32] = word;
     }
     // list bounds and the angle index
     auto bucket_start = [&](uint32_t b) { return b ? s_hist[hist_at(b - 1)] : 0u; };
@@ -380,6 +393,7 @@ int build_arc_layout(const DeviceCache& cache, uint64_t records, const ArcPlan& 
         place(&out->m, plan.entries + 16);
         place(&out->xy, plan.entries + 16);
         place(&out->index, plan.blocks.size() * kIndexWords);
+        place(&out->mask, plan.blocks.size() * kMaskPrimes * kMaskWords);
         place(&out->pos, records + 1);
     };
     lay_out();
@@ -397,7 +411,7 @@ int build_arc_layout(const DeviceCache& cache, uint64_t records, const ArcPlan& 
         if (e == cudaSuccess) {
             block_sort_kernel<<<(unsigned)plan.blocks.size(), kBlockThreads, smem, stream>>>(
                 out->blocks, plan.cap, cache.seg_off, cache.hot, cache.exact, cache.owner, out->w[0], out->w[1], out->w[2],
-                out->ang, out->part, out->src, out->m, out->xy, out->index, out->pos);
+                out->ang, out->part, out->src, out->m, out->xy, out->index, out->mask, out->pos);
             e = cudaGetLastError();
         }
     }

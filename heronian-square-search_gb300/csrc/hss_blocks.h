@@ -35,6 +35,7 @@ struct ArcBuild {
     uint32_t* m = nullptr;
     float2* xy = nullptr;
     uint32_t* index = nullptr;
+    uint32_t* mask = nullptr;
     uint16_t* pos = nullptr;
     std::vector<void*> owned;
 };

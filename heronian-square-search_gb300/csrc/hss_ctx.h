@@ -72,7 +72,7 @@ struct hss_ctx {
     uint64_t records = 0, ref_flattened = 0, ref_cached = 0;
     double prep_seconds = 0;
 
-    hss::DeviceCache dev{};
+    hss::ArcCache dev{};
     std::vector<void*> allocations;
 
     // launch buffers

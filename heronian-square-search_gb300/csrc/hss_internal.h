@@ -189,6 +189,14 @@ HSS_HD inline uint32_t part_step(uint32_t m_lo, uint32_t m_hi) { return (m_hi - 
 constexpr uint32_t kBucketShift = 25, kBuckets = 64;
 constexpr uint32_t kIndexWords = 8 * (kBuckets + 2) / 2;  // 16-bit entries, two per word
 
+// Bit sets over a block's entries: those whose root a small prime divides.
+constexpr uint32_t kMaskPrimes = 6;
+constexpr uint32_t kMaskWords = kBlockEntries / 32;
+HSS_HD constexpr uint32_t mask_prime(uint32_t i) { return i == 0 ? 7 : i == 1 ? 11 : i == 2 ? 13 : i == 3 ? 17 : i == 4 ? 19 : 23; }
+HSS_HD inline uint32_t mask_of(uint32_t p) {  // of a prime 7 <= p <= 23
+    return p == 7 ? 0u : p == 11 ? 1u : p == 13 ? 2u : p == 17 ? 3u : p == 19 ? 4u : 5u;
+}
+
 // Device-resident factor cache for one limit N (all pointers are device
 // pointers; host mirrors of seg_off / spf are kept by the owner).
 struct DeviceCache {
@@ -202,9 +210,12 @@ struct DeviceCache {
     const HotRec* pp_hot;       // prime-power values, hot form
     const __int128* pp_exact;   // prime-power values, exact (re, im) pairs
     uint32_t max_exponent;      // largest exponent covered by the prime-power table
-    // arc layout (hss_blocks.cu): blocks, and per sorted entry the three
-    // residue words (re | im << 10 | m^4 << 20 of one field), the angle and
-    // the record it comes from; pos: a record's place in its block
+};
+
+// The same with the arc layout (hss_blocks.cu): blocks, and per sorted entry the three
+// residue words (re | im << 10 | m^4 << 20 of one field), the angle and
+// the record it comes from; pos: a record's place in its block
+struct ArcCache : DeviceCache {
     const ArcBlock* blocks;
     const uint32_t* arc_index;  // kIndexWords per block
     const uint32_t* arc_w[kFields];
@@ -213,6 +224,7 @@ struct DeviceCache {
     const uint32_t* arc_src;
     const uint32_t* arc_m;      // the entry's root
     const float2* arc_xy;       // its value (positive imaginary part)
+    const uint32_t* arc_mask;   // kMaskPrimes * kMaskWords per block
     const uint16_t* pos;
     uint32_t block_cap;         // entries of the largest block
 };

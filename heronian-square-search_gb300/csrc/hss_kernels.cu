@@ -2170,13 +2170,13 @@ int arc_max_ctas_per_sm(int threads) {
     return n > 0 ? n : 1;
 }
 
-cudaError_t launch_arc_values(const DeviceCache& cache, uint32_t n_rows, const ArcBuffers& buf,
+cudaError_t launch_arc_values(const ArcCache& cache, uint32_t n_rows, const ArcBuffers& buf,
                               cudaStream_t stream) {
     if (n_rows) arc_value_kernel<<<n_rows, 64, 0, stream>>>(cache, buf);
     return cudaGetLastError();
 }
 
-cudaError_t launch_arc(const DeviceCache& cache, const ArcItem* items, uint32_t n_items, const ArcConfig& cfg,
+cudaError_t launch_arc(const ArcCache& cache, const ArcItem* items, uint32_t n_items, const ArcConfig& cfg,
                        const ArcBuffers& buf, cudaStream_t stream) {
     const size_t smem = arc_smem_bytes(cfg.threads);
     const void* fn = arc_fn(cfg.threads);
@@ -2283,7 +2283,7 @@ cudaError_t launch_exact(const DeviceCache& cache, const LaunchBuffers& buf, int
     return cudaGetLastError();
 }
 
-cudaError_t launch_arc_exact(const DeviceCache& cache, const ArcBuffers& buf, int ctas, cudaStream_t stream) {
+cudaError_t launch_arc_exact(const ArcCache& cache, const ArcBuffers& buf, int ctas, cudaStream_t stream) {
     exact_kernel<ArcBuffers><<<ctas, 128, 0, stream>>>(cache, buf);
     return cudaGetLastError();
 }

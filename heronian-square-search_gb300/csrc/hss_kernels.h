@@ -158,9 +158,9 @@ void build_arc_tables(uint8_t* out /* kArcTabBytes */);
 int arc_max_ctas_per_sm(int threads);
 
 // Values of the arc rows (one CTA per row).
-cudaError_t launch_arc_values(const DeviceCache& cache, uint32_t n_rows, const ArcBuffers& buf, cudaStream_t stream);
+cudaError_t launch_arc_values(const ArcCache& cache, uint32_t n_rows, const ArcBuffers& buf, cudaStream_t stream);
 // Persistent kernel over the arc items.
-cudaError_t launch_arc(const DeviceCache& cache, const ArcItem* items, uint32_t n_items, const ArcConfig& cfg,
+cudaError_t launch_arc(const ArcCache& cache, const ArcItem* items, uint32_t n_items, const ArcConfig& cfg,
                        const ArcBuffers& buf, cudaStream_t stream);
 // The pairs of the rest list that are not skipped, into the shared-prime queue.
 cudaError_t launch_arc_rest(const DeviceCache& cache, const ArcRest* rest, uint32_t n, const LaunchBuffers& buf,
@@ -208,7 +208,7 @@ double int32_peak_ops(int device, int sm_count, double* ms);
 // Exact work queued by the search kernels; run after them.
 cudaError_t launch_exact(const DeviceCache& cache, const LaunchBuffers& buf, int ctas, cudaStream_t stream);
 // The same for a queue that may hold terms of arc rows.
-cudaError_t launch_arc_exact(const DeviceCache& cache, const ArcBuffers& buf, int ctas, cudaStream_t stream);
+cudaError_t launch_arc_exact(const ArcCache& cache, const ArcBuffers& buf, int ctas, cudaStream_t stream);
 
 // Serving: copies a wave's row counters rows[i] into the requests' device-
 // resident state, state[slots[i]], marked done (RowCounts::pad = 1), so a
