@@ -154,6 +154,7 @@ struct ArcShared {
     uint32_t item, ahead, next;
     uint32_t pad;
     ArcBlock block;
+    ArcItem rec;  // read from here by the units, not kept in registers
 };
 
 // Asks for a block's arrays in L2 (sizes and addresses are multiples of 16 bytes).
@@ -603,6 +604,8 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ ArcC
         const uint32_t it = S.item;
         if (it >= n_items) break;
         const ArcItem w = items[it];
+        if (tid < sizeof(ArcItem) / 4)
+            reinterpret_cast<uint32_t*>(&S.rec)[tid] = reinterpret_cast<const uint32_t*>(items + it)[tid];
         if (tid < sizeof(ArcBlock) / 4)
             reinterpret_cast<uint32_t*>(&S.block)[tid] = reinterpret_cast<const uint32_t*>(cache.blocks + w.block)[tid];
         {
@@ -648,19 +651,19 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ ArcC
         const ArcBlock& B = S.block;
         const uint32_t type = B.type, block0 = B.base;
         // warps take rows (or parts of rows) on their own
-        const uint32_t shared = w.split * w.parts, units = (shared + w.nv - w.split) * w.share;
+        const uint32_t shared = S.rec.split * S.rec.parts, units = (shared + S.rec.nv - S.rec.split) * S.rec.share;
         for (;;) {
             uint32_t unit = 0;
             if (lane == 0) unit = atomicAdd(&S.next, 1u);
             unit = __shfl_sync(kFull, unit, 0);
             if (unit >= units) break;
             // of the runs of a group, this warp's: lanes = turn mod share
-            const uint32_t turn = unit % w.share;
-            const uint32_t mask_mine = kFull / ((w.share < 32 ? 1u << w.share : 0u) - 1u) << turn;  // share a power of two
-            unit /= w.share;
+            const uint32_t turn = unit % S.rec.share;
+            const uint32_t mask_mine = kFull / ((S.rec.share < 32 ? 1u << S.rec.share : 0u) - 1u) << turn;  // share a power of two
+            unit /= S.rec.share;
             const bool whole = unit >= shared;
-            const uint32_t parts = whole ? 1u : w.parts, part = whole ? 0u : unit % parts;
-            const uint32_t v = w.v0 + (whole ? unit - shared + w.split : unit / parts);
+            const uint32_t parts = whole ? 1u : S.rec.of, part = whole ? 0u : S.rec.from + unit % S.rec.parts;
+            const uint32_t v = S.rec.v0 + (whole ? unit - shared + S.rec.split : unit / S.rec.parts);
             __syncwarp();
             if (lane < sizeof(ArcRow) / 4)
                 reinterpret_cast<uint32_t*>(&T.row)[lane] = reinterpret_cast<const uint32_t*>(buf.arc_rows + v)[lane];
@@ -681,7 +684,7 @@ __global__ void __launch_bounds__(NT, 1) arc_kernel(const __grid_constant__ ArcC
                 if (lane == 0) T.row.rules = match | (defined & ~match) << 3 | (odd ? 64u : 0u) | (always ? 128u : 0u) | lt << 8;
             }
             ArcCounts counts;
-            if (!arc_prepare(cache, buf, B, w.block, s_ang, T, W.bits, W.rank, W.range, lane, counts)) continue;
+            if (!arc_prepare(cache, buf, B, S.rec.block, s_ang, T, W.bits, W.rank, W.range, lane, counts)) continue;
             const bool excl = counts.excl;
             const uint32_t k0[kFields] = {T.row.c0[0], T.row.c0[1], T.row.c0[2]};
             auto marked = [&](uint32_t i) { return ((W.bits[i >> 5] >> (i & 31u)) & 1u) != 0; };

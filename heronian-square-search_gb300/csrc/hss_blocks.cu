@@ -32,7 +32,7 @@ namespace {
 
 constexpr uint32_t kBlockThreads = 512;
 constexpr uint32_t kBlockLeast = 128;
-constexpr float kBlockScale = 9.f;
+constexpr float kBlockScale = 3.f;
 
 constexpr TypeTables kTypeTables = make_type_tables();
 __constant__ TypeTables c_types = make_type_tables();
@@ -47,8 +47,9 @@ __device__ __forceinline__ uint32_t residue_i64(int64_t v, uint32_t m) {
 // take it over its size (the warp's boundary closes one too).  The size: a row
 // pays for every run it starts in a block (less the larger the block) and for
 // every term between the tightest and the widest window of the block's roots (as
-// the square of the size over the root), so the best size grows as the square
-// root of the root.  Without `blocks` the warp's count is left in at[task], with
+// the square of the size over the root and the type's share of all roots), so the
+// best size grows as the square root of root times share (a factor of 3: 16,384
+// rows at LIMIT 10^5 132 ms, a heavy root at 10^7 23.2; of 2: 147 and 22.5, of 4.5: 129 and 23.7).  Without `blocks` the warp's count is left in at[task], with
 // them they are written from there on.  0.2 ms each time at N = 10^7, where host
 // threads took 14 ms.
 constexpr uint32_t kCutRoots = 8192;
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(kCutWarps * 32) block_cut_kernel(const uint32_
                 b.m_lo = __shfl_sync(0xFFFFFFFFu, m, from);
                 b.rank0 = r0 + from;
                 b.type = type;
-                target = min(kBlockEntries, max(kBlockLeast, (uint32_t)(kBlockScale * sqrtf((float)b.m_lo))));
+                target = min(kBlockEntries, max(kBlockLeast, (uint32_t)(kBlockScale * sqrtf((float)(c_types.count[type] * b.m_lo)))));
             }
             const bool over = lane < have && lane >= from + (b.n_m == 0) && b.n + (upto - used) > target;
             const uint32_t stop = __ballot_sync(0xFFFFFFFFu, over);

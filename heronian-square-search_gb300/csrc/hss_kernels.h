@@ -78,16 +78,19 @@ static_assert(sizeof(ArcRow) == 80, "arc row is 80 bytes");
 
 // One unit of arc work: rows v0 .. v0 + nv - 1 against one block (those whose
 // class or range leaves the block out are passed over).  Warps take whole rows,
-// except for the first `split` rows (those of many values), whose groups of
-// 32 runs are shared by `parts` warps each; where an item has too few rows for
-// its warps even so, `share` warps take every share-th run of a group.
+// except for the first `split` rows (those of many values): their groups of 32
+// runs are dealt out to `of` parts, of which the item holds `parts` from `from`
+// on (a row of very many values is shared by several items).  Where an item has
+// too few rows for its warps even so, `share` warps take every share-th run of
+// a group.
 struct ArcItem {
     uint32_t block, base;         // the block and its first entry
     uint32_t v0;
-    uint16_t nv, split, parts, n; // n: the block's entries
+    uint16_t nv, split, parts, from, of, n; // n: the block's entries
     uint32_t share;               // 1, 2, 4 or 8
+    uint32_t pad;
 };
-static_assert(sizeof(ArcItem) == 24, "arc item is 24 bytes");
+static_assert(sizeof(ArcItem) == 32, "arc item is 32 bytes");
 
 struct ArcConfig {
     int threads;      // CTA size (512 or 768)

@@ -9,6 +9,7 @@ namespace hss {
 namespace {
 
 constexpr size_t kMergedRows = 64;  // most rows of an item of several groups
+constexpr uint64_t kSmallItem = 300;    // items are not cut below this cost for balance alone (100: 2 % and up to 30 % at small limits)
 constexpr uint64_t kMergedCost = 1000;  // and their cost at most (400 and 4,000: within 2 %)
 
 using u128 = unsigned __int128;
@@ -140,6 +141,7 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
     if (rows.over() || keys_.over() || rest.over()) return false;
     if (rows.empty()) return true;
     sort();
+    if (order_.over() || sorted_.over()) return false;
     uint32_t ent = 0;
     for (size_t i = 0; i < rows.size(); ++i) {
         rows[i].ent = ent;
@@ -184,9 +186,15 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
         groups_.push_back(g);
         g0 = g1;
     }
-    // item size: the caller's, or about twelve items per resident CTA
-    const uint64_t target = std::max<uint64_t>(16, item_target ? item_target : total / ((uint64_t)ctas * 12));
-    const uint64_t merged = std::min<uint64_t>(std::max<uint64_t>(target, 400), kMergedCost);
+    // Item size: the caller's, or a sixty-fourth of a CTA's work, but not below
+    // kSmallItem unless that leaves a CTA fewer than twelve items.  With twelve items
+    // in every call the last ones ran alone, and CTAs worked 77 % of the time of 64 rows
+    // at LIMIT 10^6 (15.1 ms, now 11.6), 81 % of 16,384 rows' at 10^5 (154 ms, 132), 83 % of a
+    // heavy root's at 10^7 (25 ms, 23).
+    const uint64_t share12 = total / ((uint64_t)ctas * 12), share64 = total / ((uint64_t)ctas * 64);
+    const uint64_t target =
+        std::max<uint64_t>(16, item_target ? item_target : std::max(share64, std::min<uint64_t>(share12, kSmallItem)));
+    const uint64_t merged = std::min(std::max(target, std::min<uint64_t>(total / ctas, 400)), kMergedCost);
     Store<ArcItem>& cut = cut_;
     Store<uint32_t>& cut_lo = cut_lo_;
     auto emit = [&](ArcItem item, uint32_t b) {
@@ -241,7 +249,7 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
                     for (size_t i = 0; i < nv; ++i) units += std::min(parts, (rows[v0 + i].na + 1) / 2);
                     uint32_t share = 1;
                     for (; units < 16 && share < 8; units *= 2) share *= 2;
-                    const ArcItem item{0, 0, (uint32_t)v0, (uint16_t)nv, (uint16_t)nv, (uint16_t)parts, 0, share};
+                    const ArcItem item{0, 0, (uint32_t)v0, (uint16_t)nv, (uint16_t)nv, (uint16_t)parts, 0, (uint16_t)parts, 0, share, 0};
                     for (uint32_t b = edge[k]; b < edge[k + 1]; ++b) emit(item, b);
                 }
             }
@@ -253,6 +261,16 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
         cut.clear();
         cut_lo.clear();
         for (size_t i = g.g0; i < g.g1;) {
+            // a row above one and a half items by itself, over several (24 parts each)
+            const uint64_t several = std::min({cost(rows[i]) / target, (uint64_t)rows[i].na / 48, (uint64_t)512});
+            if (cost(rows[i]) * 2 > target * 3 && several > 1) {
+                for (uint64_t k = 0; k < several; ++k) {
+                    cut.push_back(ArcItem{0, 0, (uint32_t)i, 1, 1, 24, (uint16_t)(24 * k), (uint16_t)(24 * several), 0, 1, 0});
+                    cut_lo.push_back(rows[i].m_lo);
+                }
+                ++i;
+                continue;
+            }
             uint64_t w = 0;
             size_t e = i;
             uint32_t lo = UINT32_MAX;
@@ -266,7 +284,7 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
             // (a part holds at least a few groups of 32 runs)
             const uint64_t parts =
                 split ? std::max<uint64_t>(1, std::min({(uint64_t)24, (cost(rows[i]) * 48 + w - 1) / w, (uint64_t)rows[i].na / 2})) : 1;
-            ArcItem item{0, 0, (uint32_t)i, (uint16_t)(e - i), (uint16_t)split, (uint16_t)parts, 0, 1};
+            ArcItem item{0, 0, (uint32_t)i, (uint16_t)(e - i), (uint16_t)split, (uint16_t)parts, 0, (uint16_t)parts, 0, 1, 0};
             // fewer units than warps: the runs of a group are shared too
             uint64_t units = split * parts + (e - i - split);
             for (; units < 16 && item.share < 8; units *= 2) item.share *= 2;
@@ -278,7 +296,7 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
             for (uint32_t b = g.b0[t]; b < g.b1[t]; ++b)
                 for (size_t c = 0; c < cut.size(); ++c)
                     if (cut_lo[c] <= plan.blocks[b].m_hi) emit(cut[c], b);
-        if (items.over()) return false;
+        if (items.over() || cut.over() || cut_lo.over()) return false;
     }
     return true;
 }
