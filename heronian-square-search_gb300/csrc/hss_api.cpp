@@ -43,10 +43,14 @@ constexpr uint64_t kArcLimit = 10000;          // and long calls use it from thi
 constexpr size_t kArcRows = 64;
 constexpr uint64_t kMergedCap = 96ull << 20;   // shared-prime queue entries
 constexpr uint32_t kDescChunk = 1u << 24;       // shared-prime pairs set up per chunk (192 bytes each: 3 GB)
-// With the arc layout only the rest list's few pairs come by the shared-prime
-// kernels: small queues (0.5 GB; a plain scan enlarges them when it is called).
+// Where every search goes by arcs only the rest list's pairs come by the
+// shared-prime kernels: the queues start small (0.1 GB; opening, one search and closing at LIMIT
+// 10^7 take 23.3 ms so, 25.1 ms with the full ones of 2.4 GB) and are enlarged
+// once, when a call first needs more.
 constexpr uint64_t kArcMergedCap = 48ull << 20;
 constexpr uint32_t kArcDescChunk = 1u << 23;
+constexpr uint64_t kArcMergedStart = 2ull << 20;
+constexpr uint32_t kArcDescStart = 1u << 19;
 
 
 }  // namespace
@@ -139,22 +143,24 @@ int ensure_rows(hss_t* h, size_t rows) {
 }
 
 // Grows the shared-prime queue (entries of 16 bytes) to hold `n` pairs.
-// And a handle with the arc layout gets its whole chunk of descriptors here.
+// A handle with the arc layout starts with smaller queues: its chunk of
+// descriptors grows here too.
 int ensure_merged(hss_t* h, uint64_t n) {
-    if (n > h->desc_chunk && h->desc_chunk < kDescChunk) {
+    const uint32_t chunk = n > kArcDescChunk ? kDescChunk : kArcDescChunk;
+    if (n > h->desc_chunk && h->desc_chunk < chunk) {
         HSS_CUDA(h, cudaStreamSynchronize(h->stream));
         uint4* larger = nullptr;
-        if (int s = device_alloc(h, &larger, (size_t)kDescChunk * kBigEntryWords)) return s;
+        if (int s = device_alloc(h, &larger, (size_t)chunk * kBigEntryWords)) return s;
         device_free(h, h->d_desc);
         h->d_desc = larger;
-        h->desc_chunk = kDescChunk;
+        h->desc_chunk = chunk;
     }
     if (n <= h->merged_cap) return HSS_OK;
     if (n >= UINT32_MAX) return fail(h, HSS_ERR_OVERFLOW, "shared-prime queue beyond 32-bit indexing");
     HSS_CUDA(h, cudaStreamSynchronize(h->stream));
     device_free(h, h->d_merged);
     h->d_merged = nullptr;
-    uint64_t cap = n + n / 8;
+    uint64_t cap = std::max<uint64_t>(n + n / 8, kArcMergedCap);
     if (cap >= UINT32_MAX) cap = UINT32_MAX - 1;
     int s = device_alloc(h, &h->d_merged, (size_t)cap);
     if (s) return s;
@@ -261,9 +267,9 @@ int ensure_items(hss_t* h, size_t n) {
 // set over the same cache.
 int alloc_launch_buffers(hss_t* h) {
     h->hit_cap = h->opts.hit_capacity ? h->opts.hit_capacity : kDefaultHitCap;
-    h->merged_cap = (uint32_t)(h->plan ? kArcMergedCap : kMergedCap);
+    h->merged_cap = (uint32_t)(!h->plan ? kMergedCap : h->limit < kArcLimit ? kArcMergedCap : kArcMergedStart);
     h->big_cap = 1u << 20;
-    h->desc_chunk = h->plan ? kArcDescChunk : kDescChunk;
+    h->desc_chunk = !h->plan ? kDescChunk : h->limit < kArcLimit ? kArcDescChunk : kArcDescStart;
     h->exact_cap = h->opts.exact_capacity ? std::min<uint32_t>(h->opts.exact_capacity, 1u << 28) : 1u << 24;
     int s;
     if ((s = device_alloc(h, &h->d_hits, h->hit_cap)) || (s = device_alloc(h, &h->d_ctrl, 8)) ||
@@ -617,6 +623,8 @@ int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
         for (size_t i = start; i < start + piece; ++i) {
             h->planner.add(h->h_row_info[i], rows[i].index, h->limit, h->dev.max_exponent, 1, h->limit,
                            min_roots(h->limit, rows.size()));
+            if (h->planner.rest_pairs >= h->merged_cap / 2 && h->merged_cap < kArcMergedCap)
+                if (int s = ensure_merged(h, kArcMergedCap)) return s;
             const bool full = h->planner.entries >= kGroupValues || h->planner.rows.size() >= kGroupRows ||
                               h->planner.rest_pairs >= h->merged_cap / 2;
             if (!full && i + 1 < start + piece) continue;
