@@ -1173,13 +1173,18 @@ __global__ void __launch_bounds__(NT, MINB) batched_kernel(const DeviceCache cac
 
 // -------------------------------------------------------------- plain kernel
 
-// One block per (row, slice) and one thread per pair, as the reference
-// (gpu_search_v42.cu:298-304); events are handled by the lane that raised them.
+// One block per (row, slice), as the reference (gpu_search_v42.cu:298-304); a
+// warp takes 32 consecutive roots, a lane per pair for their constants, and
+// then lays the pairs' records end to end, a lane per record against the row's
+// values.  Events are handled by the lane that raised them.  Bound by the
+// integer work of the products; with a lane per pair throughout, a warp waited
+// for its largest pair (1,000 rows at LIMIT 5000: 7.8 ms, 1.7 ms so).
 __global__ void __launch_bounds__(kPlainThreads, 4) plain_kernel(const DeviceCache cache, uint32_t alpha_cap,
                                                                  const LaunchBuffers buf) {
     extern __shared__ __align__(16) unsigned char smem[];
     AlphaHot* s_alpha = reinterpret_cast<AlphaHot*>(smem);
     uint8_t* s_tab = reinterpret_cast<uint8_t*>(s_alpha + alpha_cap);
+    __shared__ PairCtx s_ctx[kPlainThreads];
     const uint32_t row = blockIdx.x / kSlices, slice = blockIdx.x % kSlices;
     const RowInfo& R = buf.row_info[row];
     const uint64_t l = R.l;
@@ -1189,22 +1194,46 @@ __global__ void __launch_bounds__(kPlainThreads, 4) plain_kernel(const DeviceCac
     __syncthreads();
     Acc acc{0, 0, 0, 0, 0, 0};
     const uint64_t n = cache.limit;
-    for (uint64_t m = l + slice * kPlainThreads + threadIdx.x; m <= n; m += kSlices * kPlainThreads) {
-        const uint32_t s0 = cache.seg_off[m], s1 = cache.seg_off[m + 1];
-        const uint32_t kind = classify(R, (uint32_t)m, s1 - s0 - 1);
-        if (kind == kSkip) continue;
-        acc.processed += 1;
-        if (kind == kMerged) {
-            acc.merged += 1;
-            push_merged(buf, (uint32_t)l, (uint32_t)m, row);
-            continue;
+    const uint32_t lane = threadIdx.x & 31;
+    PairCtx* ctx = s_ctx + (threadIdx.x & ~31u);  // of the warp's 32 pairs
+    for (uint64_t m0 = l + slice * kPlainThreads + (threadIdx.x & ~31u); m0 <= n; m0 += kSlices * kPlainThreads) {
+        const uint64_t m = m0 + lane;
+        uint32_t s0 = 0, len = 0;
+        if (m <= n) {
+            s0 = cache.seg_off[m];
+            const uint32_t records = cache.seg_off[m + 1] - s0;
+            const uint32_t kind = classify(R, (uint32_t)m, records - 1);
+            if (kind != kSkip) acc.processed += 1;
+            if (kind == kMerged) {
+                acc.merged += 1;
+                push_merged(buf, (uint32_t)l, (uint32_t)m, row);
+            } else if (kind != kSkip) {
+                uint32_t cc_c, cc_r;
+                ctx[lane] = make_ctx(R, m, cc_c, cc_r);
+                acc.prod += pair_products(na, records);
+                acc.cand += cc_c;
+                acc.r16 += cc_r;
+                len = records;
+            }
         }
-        uint32_t cc_c, cc_r;
-        const PairCtx c = make_ctx(R, m, cc_c, cc_r);
-        acc.prod += pair_products(na, s1 - s0);
-        acc.cand += cc_c;
-        acc.r16 += cc_r;
-        for (uint32_t j = s0; j < s1; ++j) {
+        uint32_t incl = len;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, d);
+            if (lane >= d) incl += t;
+        }
+        const uint32_t total = __shfl_sync(kFull, incl, 31), first = incl - len;
+        __syncwarp();
+        for (uint32_t q0 = 0; q0 < total; q0 += 32) {
+            const uint32_t q = q0 + lane;
+            uint32_t own = 0;  // the first pair whose inclusive sum exceeds q
+#pragma unroll
+            for (uint32_t step = 16; step; step >>= 1)
+                if (__shfl_sync(kFull, incl, own + step - 1) <= q) own += step;
+            own &= 31u;
+            const uint32_t j = __shfl_sync(kFull, s0, own) + (q - __shfl_sync(kFull, first, own));
+            if (q >= total) continue;
+            const PairCtx c = ctx[own];
             const HotRec b = cache.hot[j];
             const bool cb = (b.rre & kCentralBit) != 0;
             for (uint32_t k = 0; k < na; ++k) {
@@ -1216,6 +1245,7 @@ __global__ void __launch_bounds__(kPlainThreads, 4) plain_kernel(const DeviceCac
                                                 (uint32_t)n, &buf));
             }
         }
+        __syncwarp();
     }
     flush_acc_lanes(acc, &buf.rows[row]);
 }
