@@ -102,10 +102,12 @@ def logical_pairs(first, last, limit=LIMIT):
     return k * (limit + 1) - (first + last) * k // 2
 
 
-def model_ops(q, p, c, r):
-    """Integer-operation model of the hot path (32-bit ops): 16 per processed
-    pair, 64 per Gaussian product, 32 per candidate, 160 per mod-16 survivor."""
-    return 16 * q + 64 * p + 32 * c + 160 * r
+def model_ops(r):
+    """Integer-operation model of the hot path (32-bit ops): candidates are
+    counted by positions in sorted lists, so what grows with the work is the
+    residue filter of the mod-16 survivors, three fields of 8 operations (two
+    shifts, three multiply-adds, the table index, the lookup, the test) each."""
+    return 24 * r
 
 
 class Clocks:
@@ -507,15 +509,11 @@ def our_arm(args, rank, world, local_rank):
     lib = hss.load_library()
     peak, probe_ms = ctypes.c_double(), ctypes.c_double()
     peak_ops = peak.value if lib.hss_int32_peak(local_rank, ctypes.byref(peak), ctypes.byref(probe_ms)) == 0 else 0.0
-    q = c["processed"] - c["merged"]
-    p = c["products"] - c["merged_products"]
-    cc = c["candidates"] - c["merged_candidates"]
-    rr = c["r16"] - c["merged_r16"]
-    achieved = model_ops(q, p, cc, rr) / (main_ms * 1e-3) / 1e9
+    achieved = model_ops(c["r16"]) / (main_ms * 1e-3) / 1e9
     traffic = hbm = None
     if TRAFFIC.exists():
         t = json.loads(TRAFFIC.read_text())
-        traffic = t.get("batched_kernel_bytes_per_launch")
+        traffic = t.get("persistent_kernel_bytes_per_launch")
         if traffic and PEAKS.exists():
             # the persistent kernel's DRAM bytes of this batch (every launch of
             # it, captured on the batch itself) over its device time
@@ -538,8 +536,8 @@ def our_arm(args, rank, world, local_rank):
         "config": {"workload": f"LIMIT={LIMIT}, root edges {first}..{last} per GPU (one reference batch)",
                    "limit": LIMIT, "roots_per_gpu": ROWS, "pairs_per_gpu": pairs, "mode": "batched",
                    "parallelism": f"replicas{world}",
-                   "arithmetic": "int32 residues and f32 bounds in the filter loop; i128 exact path, u256 recheck",
-                   "l2": "inputs larger than L2: each step streams the m-side factor records (about 0.4 GB)"},
+                   "arithmetic": "int32 residues in the filter, int32 angles with f32 windows for doubtful terms; i128 exact path, u256 recheck",
+                   "l2": "inputs larger than L2: each step streams the blocks of the m-side values (about 0.6 GB)"},
         "e2e": {"value": world * pairs / (e2e_ms * 1e-3), "unit": UNIT,
                 "h2d_bytes_per_step": c["h2d_bytes"], "d2h_bytes_per_step": c["d2h_bytes"]},
         "candidates_per_s": world * c["candidates"] / (dev_ms * 1e-3),
@@ -556,7 +554,7 @@ def our_arm(args, rank, world, local_rank):
                                      "hits")},
         "roofline": {"bound": "int32", "achieved": achieved, "peak": peak_ops / 1e9, "unit": "Gop/s",
                      "frac": achieved / (peak_ops / 1e9) if peak_ops else None, "traffic": traffic,
-                     "model": "16 Q + 64 P + 32 C + 160 R over the persistent kernel's pairs",
+                     "model": "24 R: three residue fields of 8 operations per mod-16 survivor",
                      "kernel_ms": main_ms, "peak_source": "measured INT32 probe kernel (hss_int32_peak)",
                      "lane_clock_ceiling": lane_clock_ceiling(local_rank, clocks, achieved),
                      "hbm": hbm},

@@ -3,11 +3,12 @@
 // Replaces the reference's in-process boundary: Search::prepare builds the
 // factor cache (gpu_search_v42.cu:354-391), Search::run uploads it and loops
 // launch / synchronise / harvest over batches of at most 512 roots
-// (gpu_search_v42.cu:393-495).  Here the cache is built once per handle on all
-// host threads and stays resident; each search call is one launch sequence on
-// a private stream (batched: items built on the host, one persistent launch,
-// one shared-prime launch; plain: one launch per <= 512 roots), timed with
-// CUDA events, and its counters and hits are copied back once.
+// (gpu_search_v42.cu:393-495).  Here the cache and its sorted layout are built
+// once per handle on the device and stay resident; each search call is one
+// launch sequence on a private stream (batched: rows and items planned on the
+// host, one persistent launch, the shared-prime kernels for what it leaves;
+// plain: one launch per <= 512 roots), timed with CUDA events, and its counters
+// and hits are copied back once.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>
@@ -532,6 +533,9 @@ int run_products(hss_t* h, const std::vector<RowRef>& rows) {
     return HSS_OK;
 }
 
+// An item's weight in evaluations as arc cost (a row value against a block: about 2^13 terms).
+uint64_t arc_item_target(const hss_opts& o) { return o.item_target >> 13; }
+
 // Launches the batched sequence for the rows collected in h->planner: reset
 // cursors and queues, rows and items H2D, the rows' values, the persistent
 // kernel, the shared-prime kernels over the rest list (when it holds any) and
@@ -543,7 +547,7 @@ int run_planned(hss_t* h) {
     ArcConfig cfg;
     cfg.threads = h->opts.block_threads == 512 ? 512 : 768;
     cfg.ctas = h->sm_count * arc_max_ctas_per_sm(cfg.threads);
-    if (!p.finish(*h->plan, (uint32_t)cfg.ctas, h->opts.item_target >> 10)) return HSS_ERR_MEMORY;
+    if (!p.finish(*h->plan, (uint32_t)cfg.ctas, arc_item_target(h->opts))) return HSS_ERR_MEMORY;
     if (p.rows.empty()) return HSS_OK;
     const size_t rows_b = p.rows.size() * sizeof(ArcRow), rest_b = p.rest.size() * sizeof(ArcRest),
                  items_b = p.items.size() * sizeof(ArcItem);

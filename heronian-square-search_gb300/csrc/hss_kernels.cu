@@ -12,7 +12,10 @@
 // is a fourth power n^4 with m <= n <= N, gcd(l, m, n) = 1 and 5 | lmn.
 //
 // How it is computed here.  The reference multiplies every product out in
-// 128-bit arithmetic.  These kernels decide almost every product from
+// 128-bit arithmetic.  Most searches count candidates as runs of sorted values
+// instead (hss_arc.cuh, included below); what follows is the product path:
+// long calls at small limits, the plain form and the arc path's rest list.
+// These kernels decide almost every product from
 //   * residues of the product's coordinates mod 9360 and 45917, formed from
 //     per-value residues with 32-bit multiplies (exact), and
 //   * float coordinates with a proven error bound: |z| = 2 l^2 m^2 is known per
@@ -34,7 +37,7 @@
 // items from a global cursor; per item the row's values are staged in shared
 // memory, and each warp walks the m-side records of 128 roots (read from the
 // cache, coalesced) in lockstep rounds against them.  plain_kernel keeps the reference's shape
-// (a block per (row, slice), one thread per pair).  The pairs that share a
+// (a block per (row, slice)), a lane per record of 32 pairs at a time.  The pairs that share a
 // split prime (gpu_search_v42.cu:318-341) are set up by merged_setup_kernel (a
 // thread per pair, in chunks of the queue) and run by merged_kernel (a warp
 // per pair) or, when their lists exceed a warp's slice, merged_big_kernel (a

@@ -51,10 +51,13 @@ typedef struct {
     uint32_t prep_threads;    /* host threads for the cache build (0: all cores) */
     uint32_t hit_capacity;    /* device hit buffer per launch (0: 4096, as
                                  gpu_search_v42.cu:177-178) */
-    uint32_t block_threads;   /* batched CTA size: 128, 256 or 512 (0: 256) */
+    uint32_t block_threads;   /* batched CTA size: 128, 256 or 512 (0: 256); where
+                                 a search goes by arcs (LIMIT 10,000 and more, and
+                                 short calls), 512 picks 16 warps per CTA and
+                                 anything else 24 */
     uint32_t item_target;     /* batched item weight in alpha*beta evaluations
-                                 (0: 1<<23) */
-    uint32_t ctas_per_sm;     /* batched kernel variant: minimum CTAs per SM it is
+                                 (0: 1<<23; by arcs, chosen from the call's work) */
+    uint32_t ctas_per_sm;     /* product kernel variant: minimum CTAs per SM it is
                                  compiled for (128 threads: 4 or 6; 256: 2 or 3;
                                  512: 1); 0 picks 4 / 2 / 1 */
     uint32_t use_graph;       /* 1: capture each batched launch sequence in a
@@ -194,11 +197,11 @@ int hss_autotune(hss_t* h, uint64_t first, uint64_t last, hss_opts* best, hss_tu
  * the library (every GPU that loads the library holds it until the process
  * exits), its host staging is static too, and the handle's cache, stream and
  * tables (made by hss_open) are the inputs.  Limit per call: at most 64 root
- * rows (HSS_ERR_LIMIT beyond that); up to 4096 hits kept.  The array holds
- * 2^20 pairs sharing a split prime, 2^16 exact-work items and 2^13 big
- * shared-prime pairs at a time, so a call runs as several launch groups
- * when its rows need more (a row at LIMIT 10^7 has about 85,000 such pairs:
- * about 12 rows per group), and a group whose exact-work or big-pair queue
+ * rows (HSS_ERR_LIMIT beyond that); up to 4096 hits kept.  From LIMIT 1000 on
+ * the array holds 2^18 values of the call's rows, 2^18 work items and 2^16
+ * exact-work items at a time; below, 2^20 pairs sharing a split prime, 2^13 big
+ * ones and the exact-work items.  A call whose rows need more runs as several
+ * launches or launch groups, and a group whose exact-work or big-pair queue
  * fills is run again in smaller pieces (down to 64 roots of one row, then
  * HSS_ERR_OVERFLOW).  The first call on a device looks up the
  * array's device address (cudaGetSymbolAddress) and should come before any
