@@ -460,8 +460,9 @@ int search_many_locked(hss_t* h, const uint64_t* firsts, const uint64_t* lasts, 
 
 // Launches the batched sequence for a set of rows whose shared-prime pairs
 // fit the queue: reset cursor/queue, items H2D, persistent kernel, shared-prime
-// kernel.  Counters accumulate into d_rows[index].
-int run_batched_rows(hss_t* h, const RowRef* rows, size_t nrows) {
+// kernel.  Counters accumulate into d_rows[index].  pair_bound (at least those
+// pairs) sets how many shared-prime chunks are launched.
+int run_batched_rows(hss_t* h, const RowRef* rows, size_t nrows, uint64_t pair_bound) {
     // the pinned item buffer may still be read by the previous group's copy
     HSS_CUDA(h, cudaStreamSynchronize(h->stream));
     uint32_t acap = 1;
@@ -478,8 +479,6 @@ int run_batched_rows(hss_t* h, const RowRef* rows, size_t nrows) {
     int per_sm = batched_max_ctas_per_sm(cfg.threads, cfg.min_blocks, smem);
     cfg.ctas = h->sm_count * per_sm;
     LaunchBuffers b = buffers(h, 0);
-    uint64_t pair_bound = 0;  // sets how many shared-prime chunks are launched
-    for (size_t i = 0; i < nrows; ++i) pair_bound += merged_bound(h, rows[i].l);
     std::array<cudaEvent_t, 3> ev;
     if (int e = take_events(h, &ev)) return e;
     // the group's stream work: items H2D, queue resets, the three kernels.
@@ -526,7 +525,7 @@ int run_products(hss_t* h, const std::vector<RowRef>& rows) {
             ++end;
         }
         if (bound > h->merged_cap) return fail(h, HSS_ERR_OVERFLOW, "row exceeds the shared-prime queue");
-        int s = run_batched_rows(h, rows.data() + start, end - start);
+        int s = run_batched_rows(h, rows.data() + start, end - start, bound);
         if (s) return s;
         start = end;
     }
