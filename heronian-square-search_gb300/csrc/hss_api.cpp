@@ -46,7 +46,7 @@ constexpr uint64_t kMergedCap = 96ull << 20;   // shared-prime queue entries
 constexpr uint32_t kDescChunk = 1u << 24;       // shared-prime pairs set up per chunk (192 bytes each: 3 GB)
 // Where every search goes by arcs only the rest list's pairs come by the
 // shared-prime kernels: the queues start small (0.1 GB; opening, one search and closing at LIMIT
-// 10^7 take 23.3 ms so, 25.1 ms with the full ones of 2.4 GB) and are enlarged
+// 10^7 took 23.3 ms so, 25.1 ms with the full ones of 2.4 GB) and are enlarged
 // once, when a call first needs more.
 constexpr uint64_t kArcMergedCap = 48ull << 20;
 constexpr uint32_t kArcDescChunk = 1u << 23;
