@@ -36,8 +36,8 @@
 // fill its shared memory; two CTAs of 8 or 12 warps with smaller blocks were
 // slower (more runs per row).  Warps work on rows by themselves, with no barrier
 // but at a change of block.  In place of one test of every product (512 rows at
-// LIMIT 10^7, l = 7.5 10^6: 827 ms) the batch takes 114 ms; one root of branch
-// weight 625 takes 26 ms (87), 37 roots near the limit 1.8 ms (14.7).
+// LIMIT 10^7, l = 7.5 10^6: 778 ms) the batch takes 106 ms; one root of branch
+// weight 625 takes 23 ms (87), 37 roots near the limit 1.35 ms (14.7).
 
 __constant__ TypeTables c_arc_types = make_type_tables();
 

@@ -49,7 +49,8 @@ __device__ __forceinline__ uint32_t residue_i64(int64_t v, uint32_t m) {
 // every term between the tightest and the widest window of the block's roots (as
 // the square of the size over the root and the type's share of all roots), so the
 // best size grows as the square root of root times share (a factor of 3: 16,384
-// rows at LIMIT 10^5 132 ms, a heavy root at 10^7 23.2; of 2: 147 and 22.5, of 4.5: 129 and 23.7).  Without `blocks` the warp's count is left in at[task], with
+// rows at LIMIT 10^5 132 ms, a heavy root at 10^7 23.2; of 2: 147 and 22.5, of 4.5:
+// 129 and 23.7).  Without `blocks` the warp's count is left in at[task], with
 // them they are written from there on.  0.2 ms each time at N = 10^7, where host
 // threads took 14 ms.
 constexpr uint32_t kCutRoots = 8192;
@@ -123,7 +124,9 @@ __global__ void __launch_bounds__(kCutWarps * 32) block_cut_kernel(const uint32_
 //      than one key on average, and equal ones are ordered by record), then the
 //      sorted arrays' entry.  Central values need no sort: their place is the
 //      root's rank.
-// Bound by the records' reads and the entries' writes (36 and 35 bytes).  A
+// 36 bytes read and 35 written per value, 1.2 TB/s: what bounds it is its barriers
+// and chains of shared-memory accesses (26 % of the DRAM rate, 35 % of the issue
+// slots, at N = 10^6), two CTAs per SM.  A
 // bitonic sort of (key, record) pairs in shared memory, with a thread per root
 // for the keys, took 11.5 ms at N = 10^7; this form takes 5.5 ms.
 constexpr uint32_t kFine = 1024;
