@@ -94,6 +94,40 @@ void device_free(hss_t* h, void* p) {
     cudaFree(p);
 }
 
+// Replaces an array of *cap elements (of `per` T each) by one of n.  Where it
+// cannot be had the old one stays: memory for both being short, the old one is
+// given up first and allocated again if that was not enough.  Only where that
+// fails too is the array gone, and its capacity 0: no capacity ever claims
+// more than its array holds.
+template <class T, class Cap>
+int device_grow(hss_t* h, T** p, Cap* cap, size_t n, size_t per = 1) {
+    T* larger = nullptr;
+    int s = device_alloc(h, &larger, n * per);
+    if (s && *cap) {
+        const size_t old = *cap;
+        device_free(h, *p);
+        *p = nullptr;
+        *cap = 0;
+        if ((s = device_alloc(h, &larger, n * per)) && device_alloc(h, p, old * per) == HSS_OK) *cap = (Cap)old;
+    }
+    if (s) return s;
+    device_free(h, *p);
+    *p = larger;
+    *cap = (Cap)n;
+    return HSS_OK;
+}
+
+// The same for pinned host memory, whose contents are not kept.
+template <class T>
+int host_grow(hss_t* h, T** p, size_t* cap, size_t n) {
+    if (*p) cudaFreeHost(*p);
+    *p = nullptr;
+    *cap = 0;
+    HSS_CUDA(h, cudaMallocHost(p, n * sizeof(T)));
+    *cap = n;
+    return HSS_OK;
+}
+
 template <class T>
 int upload(hss_t* h, T** out, const T* src, size_t count) {
     int s = device_alloc(h, out, count);
@@ -129,17 +163,11 @@ uint64_t merged_bound(const hss_t* h, uint64_t l) {
 }
 
 int ensure_rows(hss_t* h, size_t rows) {
-    if (rows <= h->rows_cap) return HSS_OK;
-    device_free(h, h->d_rows);
-    h->d_rows = nullptr;
-    size_t cap = std::max(rows, (size_t)1024);
-    int s = device_alloc(h, &h->d_rows, cap);
-    if (s) return s;
-    h->rows_cap = cap;
-    if (h->h_rows) cudaFreeHost(h->h_rows);
-    h->h_rows = nullptr;
-    HSS_CUDA(h, cudaMallocHost(&h->h_rows, cap * sizeof(RowCounts)));
-    h->h_rows_cap = cap;
+    const size_t cap = std::max(rows, (size_t)1024);
+    if (rows > h->rows_cap)
+        if (int s = device_grow(h, &h->d_rows, &h->rows_cap, cap)) return s;
+    if (rows > h->h_rows_cap)
+        if (int s = host_grow(h, &h->h_rows, &h->h_rows_cap, cap)) return s;
     return HSS_OK;
 }
 
@@ -150,23 +178,14 @@ int ensure_merged(hss_t* h, uint64_t n) {
     const uint32_t chunk = n > kArcDescChunk ? kDescChunk : kArcDescChunk;
     if (n > h->desc_chunk && h->desc_chunk < chunk) {
         HSS_CUDA(h, cudaStreamSynchronize(h->stream));
-        uint4* larger = nullptr;
-        if (int s = device_alloc(h, &larger, (size_t)chunk * kBigEntryWords)) return s;
-        device_free(h, h->d_desc);
-        h->d_desc = larger;
-        h->desc_chunk = chunk;
+        if (int s = device_grow(h, &h->d_desc, &h->desc_chunk, chunk, kBigEntryWords)) return s;
     }
     if (n <= h->merged_cap) return HSS_OK;
     if (n >= UINT32_MAX) return fail(h, HSS_ERR_OVERFLOW, "shared-prime queue beyond 32-bit indexing");
     HSS_CUDA(h, cudaStreamSynchronize(h->stream));
-    device_free(h, h->d_merged);
-    h->d_merged = nullptr;
     uint64_t cap = std::max<uint64_t>(n + n / 8, kArcMergedCap);
     if (cap >= UINT32_MAX) cap = UINT32_MAX - 1;
-    int s = device_alloc(h, &h->d_merged, (size_t)cap);
-    if (s) return s;
-    h->merged_cap = (uint32_t)cap;
-    return HSS_OK;
+    return device_grow(h, &h->d_merged, &h->merged_cap, (size_t)cap);
 }
 
 // A launch group whose exact work outgrew the exact queue, or whose big
@@ -180,19 +199,13 @@ int grow_overflowed(hss_t* h) {
         h->exact_overflow = false;
         const uint64_t cap = (uint64_t)h->exact_cap * 4;
         if (cap > (1ull << 28)) return HSS_ERR_OVERFLOW;
-        device_free(h, h->d_exact);
-        h->d_exact = nullptr;
-        if (int s = device_alloc(h, &h->d_exact, (size_t)cap)) return s;
-        h->exact_cap = (uint32_t)cap;
+        if (int s = device_grow(h, &h->d_exact, &h->exact_cap, (size_t)cap)) return s;
     }
     if (h->big_overflow) {
         h->big_overflow = false;
         const uint64_t cap = (uint64_t)h->big_cap * 4;
         if (cap > (1ull << 24)) return HSS_ERR_OVERFLOW;
-        device_free(h, h->d_big);
-        h->d_big = nullptr;
-        if (int s = device_alloc(h, &h->d_big, (size_t)cap * kBigEntryWords)) return s;
-        h->big_cap = (uint32_t)cap;
+        if (int s = device_grow(h, &h->d_big, &h->big_cap, (size_t)cap, kBigEntryWords)) return s;
     }
     return HSS_OK;
 }
@@ -244,21 +257,25 @@ int ensure_group(hss_t* h, size_t bytes, size_t values) {
 }
 
 int ensure_items(hss_t* h, size_t n) {
-    if (n > h->items_cap) {
-        device_free(h, h->d_items);
-        h->d_items = nullptr;
-        size_t cap = std::max(n + n / 4, (size_t)1 << 16);
-        int s = device_alloc(h, &h->d_items, cap);
-        if (s) return s;
-        h->items_cap = cap;
-    }
-    if (n > h->h_items_cap) {
-        if (h->h_items) cudaFreeHost(h->h_items);
-        h->h_items = nullptr;
-        size_t cap = std::max(n + n / 4, (size_t)1 << 16);
-        HSS_CUDA(h, cudaMallocHost(&h->h_items, cap * sizeof(WorkItem)));
-        h->h_items_cap = cap;
-    }
+    const size_t cap = std::max(n + n / 4, (size_t)1 << 16);
+    if (n > h->items_cap)
+        if (int s = device_grow(h, &h->d_items, &h->items_cap, cap)) return s;
+    if (n > h->h_items_cap)
+        if (int s = host_grow(h, &h->h_items, &h->h_items_cap, cap)) return s;
+    return HSS_OK;
+}
+
+// The shared-prime, big-pair, descriptor and exact-work queues at their first
+// size, those that are not there (at open, or after a growth that lost one).
+int ensure_queues(hss_t* h) {
+    const uint64_t merged = !h->plan ? kMergedCap : h->limit < kArcLimit ? kArcMergedCap : kArcMergedStart;
+    const uint32_t chunk = !h->plan ? kDescChunk : h->limit < kArcLimit ? kArcDescChunk : kArcDescStart;
+    const uint32_t exact = h->opts.exact_capacity ? std::min<uint32_t>(h->opts.exact_capacity, 1u << 28) : 1u << 24;
+    int s = HSS_OK;
+    if (!h->merged_cap && (s = device_grow(h, &h->d_merged, &h->merged_cap, merged))) return s;
+    if (!h->big_cap && (s = device_grow(h, &h->d_big, &h->big_cap, 1u << 20, kBigEntryWords))) return s;
+    if (!h->desc_chunk && (s = device_grow(h, &h->d_desc, &h->desc_chunk, chunk, kBigEntryWords))) return s;
+    if (!h->exact_cap && (s = device_grow(h, &h->d_exact, &h->exact_cap, exact))) return s;
     return HSS_OK;
 }
 
@@ -268,16 +285,9 @@ int ensure_items(hss_t* h, size_t n) {
 // set over the same cache.
 int alloc_launch_buffers(hss_t* h) {
     h->hit_cap = h->opts.hit_capacity ? h->opts.hit_capacity : kDefaultHitCap;
-    h->merged_cap = (uint32_t)(!h->plan ? kMergedCap : h->limit < kArcLimit ? kArcMergedCap : kArcMergedStart);
-    h->big_cap = 1u << 20;
-    h->desc_chunk = !h->plan ? kDescChunk : h->limit < kArcLimit ? kArcDescChunk : kArcDescStart;
-    h->exact_cap = h->opts.exact_capacity ? std::min<uint32_t>(h->opts.exact_capacity, 1u << 28) : 1u << 24;
     int s;
     if ((s = device_alloc(h, &h->d_hits, h->hit_cap)) || (s = device_alloc(h, &h->d_ctrl, 8)) ||
-        (s = device_alloc(h, &h->d_merged, h->merged_cap)) ||
-        (s = device_alloc(h, &h->d_big, (size_t)h->big_cap * kBigEntryWords)) ||
-        (s = device_alloc(h, &h->d_desc, (size_t)h->desc_chunk * kBigEntryWords)) ||
-        (s = device_alloc(h, &h->d_exact, h->exact_cap)) || (s = ensure_rows(h, 1024)))
+        (s = ensure_queues(h)) || (s = ensure_rows(h, 1024)))
         return s;
     if ((!h->stream && cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) ||
         cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
@@ -383,16 +393,11 @@ size_t build_items(hss_t* h, const RowRef* rows, size_t nrows, uint32_t* alpha_c
 // Room for the constants of a call's rows; the stream is idle afterwards.
 int ensure_row_info(hss_t* h, size_t rows) {
     HSS_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (rows <= h->row_info_cap) return HSS_OK;
-    device_free(h, h->d_row_info);
-    h->d_row_info = nullptr;
-    if (h->h_row_info) cudaFreeHost(h->h_row_info);
-    h->h_row_info = nullptr;
-    size_t cap = std::max(rows, (size_t)1024);
-    int s = device_alloc(h, &h->d_row_info, cap);
-    if (s) return s;
-    HSS_CUDA(h, cudaMallocHost(&h->h_row_info, cap * sizeof(RowInfo)));
-    h->row_info_cap = cap;
+    const size_t cap = std::max(rows, (size_t)1024);
+    if (rows > h->row_info_cap)
+        if (int s = device_grow(h, &h->d_row_info, &h->row_info_cap, cap)) return s;
+    if (rows > h->h_row_info_cap)
+        if (int s = host_grow(h, &h->h_row_info, &h->h_row_info_cap, cap)) return s;
     return HSS_OK;
 }
 
@@ -671,6 +676,7 @@ int run_plain(hss_t* h, uint64_t first, uint64_t last) {
 
 int begin_call(hss_t* h, size_t rows) {
     int s = ensure_rows(h, rows);
+    if (!s) s = ensure_queues(h);
     if (s) return s;
     HSS_CUDA(h, cudaMemsetAsync(h->d_rows, 0, rows * sizeof(RowCounts), h->stream));
     HSS_CUDA(h, cudaMemsetAsync(h->d_ctrl, 0, 8 * sizeof(unsigned int), h->stream));
@@ -1284,16 +1290,11 @@ hss_t* make_lane(hss_t* h, int* status) {
 }
 
 int ensure_slots(hss_t* lane, size_t n) {
-    if (n <= lane->slots_cap) return HSS_OK;
-    device_free(lane, lane->d_slots);
-    lane->d_slots = nullptr;
-    if (lane->h_slots) cudaFreeHost(lane->h_slots);
-    lane->h_slots = nullptr;
     const size_t cap = std::max(n, (size_t)1024);
-    int s = device_alloc(lane, &lane->d_slots, cap);
-    if (s) return s;
-    HSS_CUDA(lane, cudaMallocHost(&lane->h_slots, cap * sizeof(uint32_t)));
-    lane->slots_cap = cap;
+    if (n > lane->slots_cap)
+        if (int s = device_grow(lane, &lane->d_slots, &lane->slots_cap, cap)) return s;
+    if (n > lane->h_slots_cap)
+        if (int s = host_grow(lane, &lane->h_slots, &lane->h_slots_cap, cap)) return s;
     return HSS_OK;
 }
 

@@ -118,7 +118,7 @@ struct hss_ctx {
     size_t h_rows_cap = 0;
     hss::RowInfo* d_row_info = nullptr;  // constants of the call's rows
     hss::RowInfo* h_row_info = nullptr;  // pinned
-    size_t row_info_cap = 0;
+    size_t row_info_cap = 0, h_row_info_cap = 0;
 
     std::mutex gpu_mu;  // serialises device work on the handle
 
@@ -153,6 +153,6 @@ struct hss_ctx {
     unsigned int* h_ctrl = nullptr;
     uint32_t* d_slots = nullptr;
     uint32_t* h_slots = nullptr;
-    size_t slots_cap = 0;
+    size_t slots_cap = 0, h_slots_cap = 0;
 };
 
