@@ -63,11 +63,15 @@ int fail(hss_t* h, int status, const std::string& msg) {
     return status;
 }
 
-#define HSS_CUDA(h, call)                                                                      \
-    do {                                                                                       \
-        cudaError_t e_ = (call);                                                               \
-        if (e_ != cudaSuccess)                                                                 \
-            return fail(h, HSS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+// (a refused call's error also stays with the thread until it is read, and the
+// check behind the next kernel launch would report it: it is taken out here)
+#define HSS_CUDA(h, call)                                                                          \
+    do {                                                                                           \
+        cudaError_t e_ = (call);                                                                   \
+        if (e_ != cudaSuccess) {                                                                   \
+            cudaGetLastError();                                                                    \
+            return fail(h, HSS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));      \
+        }                                                                                          \
     } while (0)
 
 uint64_t now_ns() {
@@ -81,7 +85,10 @@ int device_alloc(hss_t* h, T** out, size_t count) {
     void* p = nullptr;
     if (count == 0) count = 1;
     cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-    if (e != cudaSuccess) return fail(h, HSS_ERR_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(h, HSS_ERR_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     h->allocations.push_back(p);
     *out = static_cast<T*>(p);
     return HSS_OK;
@@ -1279,7 +1286,10 @@ hss_t* make_lane(hss_t* h, int* status) {
     lane->d_arc_tabs = h->d_arc_tabs;
     lane->plan = h->plan;
     int s = alloc_launch_buffers(lane);
-    if (!s && cudaMallocHost(&lane->h_ctrl, 8 * sizeof(unsigned int)) != cudaSuccess) s = HSS_ERR_MEMORY;
+    if (!s && cudaMallocHost(&lane->h_ctrl, 8 * sizeof(unsigned int)) != cudaSuccess) {
+        cudaGetLastError();
+        s = HSS_ERR_MEMORY;
+    }
     if (s) {
         hss_close(lane);
         *status = s;

@@ -344,6 +344,7 @@ int plan_arc_blocks(const uint32_t* d_seg_off, uint64_t limit, cudaStream_t stre
     cudaFree(d_at);
     cudaFree(d_blocks);
     if (e != cudaSuccess) {
+        cudaGetLastError();  // not left for the next launch's check
         *err = cudaGetErrorString(e);
         return HSS_ERR_CUDA;
     }
@@ -422,6 +423,7 @@ int build_arc_layout(const DeviceCache& cache, uint64_t records, const ArcPlan& 
     if (e != cudaSuccess) {
         for (void* p : out->owned) cudaFree(p);
         out->owned.clear();
+        cudaGetLastError();
         *err = cudaGetErrorString(e);
         return HSS_ERR_CUDA;
     }

@@ -494,6 +494,7 @@ int build_device_cache(uint64_t n, int sm_count, CUstream_st* st, DeviceBuild* o
     };
     auto fail = [&](cudaError_t e) {
         release();
+        cudaGetLastError();  // a refused allocation's error is not left for the next launch's check
         *err = cudaGetErrorString(e);
         return HSS_ERR_CUDA;
     };

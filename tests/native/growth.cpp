@@ -49,6 +49,7 @@ void check_growth(const char* what, Grow grow) {
             CHECK(s == HSS_OK || s == HSS_ERR_MEMORY || s == HSS_ERR_CUDA, "%s: status %d", what, s);
             if (k == 0 && count == 1000) CHECK(s != HSS_OK, "%s: a refused growth reported as done", what);
             check_buffers(h, what, k);
+            CHECK(fake::last == cudaSuccess, "%s, refusal %d: the next launch's check would meet its error", what, k);
             fake::reset();
             CHECK(begin_call(h, kSmall) == HSS_OK, "%s: the next call", what);
             CHECK(h->d_merged && h->merged_cap && h->d_big && h->big_cap && h->d_desc && h->desc_chunk && h->d_exact && h->exact_cap,
