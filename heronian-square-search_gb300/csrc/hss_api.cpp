@@ -47,7 +47,8 @@ constexpr uint32_t kDescChunk = 1u << 24;       // shared-prime pairs set up per
 // Where every search goes by arcs only the rest list's pairs come by the
 // shared-prime kernels: the queues start small (0.1 GB; opening, one search and closing at LIMIT
 // 10^7 took 23.3 ms so, 25.1 ms with the full ones of 2.4 GB) and are enlarged
-// once, when a call first needs more.
+// to the full ones when a call first needs more (a plain scan may need more still).
+// Where there is no room the call goes on with what there is, in smaller launches.
 constexpr uint64_t kArcMergedCap = 48ull << 20;
 constexpr uint32_t kArcDescChunk = 1u << 23;
 constexpr uint64_t kArcMergedStart = 2ull << 20;
@@ -180,19 +181,23 @@ int ensure_rows(hss_t* h, size_t rows) {
 
 // Grows the shared-prime queue (entries of 16 bytes) to hold `n` pairs.
 // A handle with the arc layout starts with smaller queues: its chunk of
-// descriptors grows here too.
+// descriptors grows here too, where there is room (the pairs of a queue are set
+// up in as many chunks as it takes).
 int ensure_merged(hss_t* h, uint64_t n) {
-    const uint32_t chunk = n > kArcDescChunk ? kDescChunk : kArcDescChunk;
+    const uint32_t chunk = n > kArcMergedCap ? kDescChunk : kArcDescChunk;
     if (n > h->desc_chunk && h->desc_chunk < chunk) {
         HSS_CUDA(h, cudaStreamSynchronize(h->stream));
-        if (int s = device_grow(h, &h->d_desc, &h->desc_chunk, chunk, kBigEntryWords)) return s;
+        const int s = device_grow(h, &h->d_desc, &h->desc_chunk, chunk, kBigEntryWords);
+        if (s && !h->desc_chunk) return s;
     }
     if (n <= h->merged_cap) return HSS_OK;
     if (n >= UINT32_MAX) return fail(h, HSS_ERR_OVERFLOW, "shared-prime queue beyond 32-bit indexing");
     HSS_CUDA(h, cudaStreamSynchronize(h->stream));
-    uint64_t cap = std::max<uint64_t>(n + n / 8, kArcMergedCap);
+    uint64_t cap = n <= kArcMergedCap ? kArcMergedCap : n + n / 8;
     if (cap >= UINT32_MAX) cap = UINT32_MAX - 1;
-    return device_grow(h, &h->d_merged, &h->merged_cap, (size_t)cap);
+    int s = device_grow(h, &h->d_merged, &h->merged_cap, (size_t)cap);
+    if (s && cap > n) s = device_grow(h, &h->d_merged, &h->merged_cap, (size_t)n);
+    return s;
 }
 
 // A launch group whose exact work outgrew the exact queue, or whose big
@@ -631,6 +636,7 @@ int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
     if (!h->plan || (h->limit < kArcLimit && rows.size() > kArcRows)) return run_products(h, rows);
     h->planner.clear();
     size_t start = 0;
+    bool grown = false;
     if (int s = ensure_row_info(h, rows.size())) return s;
     while (start < rows.size()) {
         const size_t piece = start == 0 && rows.size() >= kLongCall && !h->opts.use_graph ? rows.size() / 8 : rows.size() - start;
@@ -638,8 +644,12 @@ int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
         for (size_t i = start; i < start + piece; ++i) {
             h->planner.add(h->h_row_info[i], rows[i].index, h->limit, h->dev.max_exponent, 1, h->limit,
                            min_roots(h->limit, rows.size()));
-            if (h->planner.rest_pairs >= h->merged_cap / 2 && h->merged_cap < kArcMergedCap)
-                if (int s = ensure_merged(h, kArcMergedCap)) return s;
+            if (h->planner.rest_pairs >= h->merged_cap / 2 && h->merged_cap < kArcMergedCap && !grown) {
+                // (once a call: without room for it the groups are smaller)
+                grown = true;
+                const int s = ensure_merged(h, kArcMergedCap);
+                if (s && (s != HSS_ERR_MEMORY || !h->merged_cap || !h->desc_chunk)) return s;
+            }
             const bool full = h->planner.entries >= kGroupValues || h->planner.rows.size() >= kGroupRows ||
                               h->planner.rest_pairs >= h->merged_cap / 2;
             if (!full && i + 1 < start + piece) continue;
@@ -654,15 +664,21 @@ int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
 }
 
 int run_plain(hss_t* h, uint64_t first, uint64_t last) {
-    for (uint64_t b = first; b <= last; b += kPlainBatch) {
-        uint32_t nrows = (uint32_t)std::min<uint64_t>(kPlainBatch, last - b + 1);
+    uint32_t nrows = 0;
+    for (uint64_t b = first; b <= last; b += nrows) {
+        nrows = (uint32_t)std::min<uint64_t>(kPlainBatch, last - b + 1);
         uint64_t bound = 0;
         uint32_t acap = 1;
         for (uint64_t l = b; l < b + nrows; ++l) {
             bound += merged_bound(h, l);
             acap = std::max(acap, free_count(h, l) + 1);
         }
-        if (int g = ensure_merged(h, bound)) return g;
+        if (int s = ensure_merged(h, bound)) {
+            // without room for the batch's pairs: as many of its rows as fit, at least one
+            if (s != HSS_ERR_MEMORY || !h->merged_cap || !h->desc_chunk) return s;
+            while (nrows > 1 && bound > h->merged_cap) bound -= merged_bound(h, b + --nrows);
+            if (bound > h->merged_cap && (s = ensure_merged(h, bound))) return s;
+        }
         HSS_CUDA(h, cudaMemsetAsync(h->d_ctrl + 1, 0, sizeof(unsigned int), h->stream));
         HSS_CUDA(h, cudaMemsetAsync(h->d_ctrl + 4, 0, 3 * sizeof(unsigned int), h->stream));
         LaunchBuffers buf = buffers(h, b - first);

@@ -57,3 +57,36 @@ def test_noalloc_equals_batched(limit, first, last):
             got = s.search_noalloc(first, last)
             assert {k: got.counts[k] for k in FIELDS} == {k: want.counts[k] for k in FIELDS}
             assert got.hits == want.hits
+
+
+@pytest.fixture(scope="module")
+def plain_long():
+    with hss.Search(100_000) as s:
+        r = s.search(1, 30_000, mode="plain", rows=True)
+    return r
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["stream", "graph", "serving"])
+def test_queues_grow_from_their_first_size(plain_long, form):
+    """A long call from low roots at LIMIT 100,000, whose shared-prime pairs outgrow the 2 M entries a queue starts
+    with: by a handle, under a graph, and by a serving lane (one wave of up to 41,943 rows)."""
+    torch = pytest.importorskip("torch")
+    with hss.Search(100_000, use_graph=int(form == "graph")) as s:
+        before = torch.cuda.mem_get_info()[0]
+        if form == "serving":
+            s.serve_start(wave_mpairs=4_000)
+            before = torch.cuda.mem_get_info()[0]
+            done = s.wait(s.submit(1, 30_000))
+            counts, hits = done["counts"], done["hits"]
+        else:
+            got = s.search(1, 30_000, rows=True)
+            counts, hits = got.counts, got.hits
+            assert got.row_candidates == plain_long.row_candidates
+        grown = before - torch.cuda.mem_get_info()[0]
+    # the larger queue and its descriptors, 48 Mi entries of 16 bytes and 8 Mi of 192, in place of the first ones of
+    # 2 Mi and 0.5 Mi; not 3 GB of descriptors, and the rows, items and values of the call beside them
+    larger = 48 * 16 + 8 * 192 - (2 * 16 + 96)
+    assert larger <= grown / 2 ** 20 < larger + 1024
+    assert {k: counts[k] for k in FIELDS} == {k: plain_long.counts[k] for k in FIELDS}
+    assert sorted(hits) == sorted(plain_long.hits)
