@@ -297,9 +297,9 @@ int ensure_queues(hss_t* h) {
 // set over the same cache.
 int alloc_launch_buffers(hss_t* h) {
     h->hit_cap = h->opts.hit_capacity ? h->opts.hit_capacity : kDefaultHitCap;
-    int s;
-    if ((s = device_alloc(h, &h->d_hits, h->hit_cap)) || (s = device_alloc(h, &h->d_ctrl, 8)) ||
-        (s = ensure_queues(h)) || (s = ensure_rows(h, 1024)))
+    int s = HSS_OK;
+    if ((!h->d_hits && (s = device_alloc(h, &h->d_hits, h->hit_cap))) ||
+        (!h->d_ctrl && (s = device_alloc(h, &h->d_ctrl, 8))) || (s = ensure_queues(h)) || (s = ensure_rows(h, 1024)))
         return s;
     if ((!h->stream && cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) ||
         cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
@@ -784,6 +784,8 @@ void copy_hits(const std::vector<DevHit>& in, hss_hit* out, uint32_t cap) {
 }
 
 // The arc layout of the handle's cache (h->dev, h->records), enqueued on the stream.
+// It takes as much memory again as the cache: where the device has no room for it,
+// the handle goes without and searches by products.
 int open_arc_layout(hss_t* h) {
     if (h->limit < kArcLeast) return HSS_OK;
     auto plan = std::make_shared<ArcPlan>();
@@ -791,6 +793,7 @@ int open_arc_layout(hss_t* h) {
     std::string err;
     int s = plan_arc_blocks(h->dev.seg_off, h->limit, h->stream, plan.get(), &err);
     if (!s) s = build_arc_layout(h->dev, h->records, *plan, h->stream, &b, &err);
+    if (s == HSS_ERR_MEMORY) return HSS_OK;
     if (s) return fail(h, s, err);
     h->allocations.insert(h->allocations.end(), b.owned.begin(), b.owned.end());
     h->dev.blocks = b.blocks;
@@ -806,6 +809,26 @@ int open_arc_layout(hss_t* h) {
     h->dev.block_cap = plan->cap;
     h->plan = std::move(plan);
     return HSS_OK;
+}
+
+// The handle's launch buffers; where the layout leaves no room for them, in its place.
+int open_launch_buffers(hss_t* h) {
+    const int s = alloc_launch_buffers(h);
+    if (s != HSS_ERR_MEMORY || !h->plan) return s;
+    HSS_CUDA(h, cudaStreamSynchronize(h->stream));
+    device_free(h, const_cast<ArcBlock*>(h->dev.blocks));  // the first array of the layout's one allocation
+    h->plan.reset();
+    // (the product path's queues are larger)
+    auto drop = [&](auto** p, uint32_t* cap) {
+        device_free(h, *p);
+        *p = nullptr;
+        *cap = 0;
+    };
+    drop(&h->d_merged, &h->merged_cap);
+    drop(&h->d_big, &h->big_cap);
+    drop(&h->d_desc, &h->desc_chunk);
+    drop(&h->d_exact, &h->exact_cap);
+    return alloc_launch_buffers(h);
 }
 
 }  // namespace
@@ -1002,7 +1025,7 @@ int hss_open(uint64_t limit, int device, const hss_opts* opts, hss_t** out) {
     std::vector<uint8_t> arc_tabs(kArcTabBytes);
     build_arc_tables(arc_tabs.data());
     if ((s = upload(h, &h->d_tables, tables.data(), kTableTotalBytes)) ||
-        (s = upload(h, &h->d_arc_tabs, arc_tabs.data(), kArcTabBytes)) || (s = alloc_launch_buffers(h))) {
+        (s = upload(h, &h->d_arc_tabs, arc_tabs.data(), kArcTabBytes)) || (s = open_launch_buffers(h))) {
         hss_close(h);
         return s;
     }

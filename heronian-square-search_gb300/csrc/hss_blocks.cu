@@ -346,7 +346,7 @@ int plan_arc_blocks(const uint32_t* d_seg_off, uint64_t limit, cudaStream_t stre
     if (e != cudaSuccess) {
         cudaGetLastError();  // not left for the next launch's check
         *err = cudaGetErrorString(e);
-        return HSS_ERR_CUDA;
+        return e == cudaErrorMemoryAllocation ? HSS_ERR_MEMORY : HSS_ERR_CUDA;
     }
     uint64_t base = 0;
     plan->cap = 0;
@@ -425,7 +425,7 @@ int build_arc_layout(const DeviceCache& cache, uint64_t records, const ArcPlan& 
         out->owned.clear();
         cudaGetLastError();
         *err = cudaGetErrorString(e);
-        return HSS_ERR_CUDA;
+        return e == cudaErrorMemoryAllocation ? HSS_ERR_MEMORY : HSS_ERR_CUDA;
     }
     return HSS_OK;
 }

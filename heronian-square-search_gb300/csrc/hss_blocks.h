@@ -23,6 +23,7 @@ struct ArcPlan {
 
 // Cuts the roots 1..limit of every type into blocks of at most kBlockEntries
 // records (on the device, from its segment offsets; waits for the stream).
+// This and build_arc_layout return HSS_ERR_MEMORY where the device has no room.
 int plan_arc_blocks(const uint32_t* d_seg_off, uint64_t limit, cudaStream_t stream, ArcPlan* plan, std::string* err);
 
 // Device arrays of the arc layout; `owned` lists the allocations.

@@ -128,7 +128,10 @@ const char* hss_last_error(const hss_t* h);
 /* Builds the Gaussian factor cache for LIMIT resident on `device`, by
  * kernels on the device or (opts->host_build) on the host and uploaded
  * (replaces Search::prepare and the uploads of Search::run,
- * gpu_search_v42.cu:354-432).  1 <= limit <= HSS_MAX_LIMIT. */
+ * gpu_search_v42.cu:354-432).  1 <= limit <= HSS_MAX_LIMIT.  From LIMIT 1000 on
+ * the cache's values are laid out a second time, sorted, for the searches by
+ * arcs; where the device has no room for that the handle opens without and
+ * searches by products (same results, several times slower). */
 int hss_open(uint64_t limit, int device, const hss_opts* opts, hss_t** out);
 
 /* Releases the device cache and the handle (gpu_search_v42.cu:496-505). */
