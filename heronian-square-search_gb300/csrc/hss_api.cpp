@@ -563,7 +563,9 @@ int run_planned(hss_t* h) {
     ArcConfig cfg;
     cfg.threads = h->opts.block_threads == 512 ? 512 : 768;
     cfg.ctas = h->sm_count * arc_max_ctas_per_sm(cfg.threads);
-    if (!p.finish(*h->plan, (uint32_t)cfg.ctas, arc_item_target(h->opts))) return HSS_ERR_MEMORY;
+    if (p.entries > kArcValuesMost) return fail(h, HSS_ERR_OVERFLOW, "a launch group's values beyond 25-bit numbering");
+    if (!p.finish(*h->plan, (uint32_t)cfg.ctas, arc_item_target(h->opts)))
+        return fail(h, HSS_ERR_MEMORY, "no memory for a launch group's rows and items");
     if (p.rows.empty()) return HSS_OK;
     const size_t rows_b = p.rows.size() * sizeof(ArcRow), rest_b = p.rest.size() * sizeof(ArcRest),
                  items_b = p.items.size() * sizeof(ArcItem);
@@ -621,7 +623,8 @@ int run_planned(hss_t* h) {
 // Splits the call's rows into launch groups whose values and rest pairs fit the
 // buffers.  Of a long call the first eighth is a group by itself, so that the
 // device works while the host plans the rest.
-constexpr uint64_t kGroupValues = 8ull << 20;
+constexpr uint64_t kGroupValues = 8ull << 20;  // and one root more: 13.3 M at most, for 15,413,645 at LIMIT 3 10^7
+static_assert(kGroupValues + (13ull << 20) <= kArcValuesMost, "a group's values can be numbered");
 constexpr size_t kGroupRows = 1u << 20;
 constexpr size_t kLongCall = 2048;
 

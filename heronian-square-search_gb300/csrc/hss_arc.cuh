@@ -121,6 +121,7 @@ __device__ __forceinline__ uint32_t arc_test(const uint32_t* x, const ArcFilter&
 // A staged run: words 0..2 and 4..6 the first two multipliers of the fields,
 // word 8 its value and form (kRunId) and these marks, 9 its angle, 10 and 11 its bounds
 // p0 | c0 << 16 and c1 | p1 << 16.
+static_assert(kArcValuesMost << 3 == 1ull << 28, "a value and its form fit kRunId");
 constexpr uint32_t kRunId = 0x0FFFFFFFu, kRunCentral = 1u << 28, kRunLower = 1u << 29, kRunKeep = 1u << 30;
 
 // A row against the CTA's block, as one warp works on it.

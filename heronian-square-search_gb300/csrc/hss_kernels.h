@@ -92,6 +92,9 @@ struct ArcItem {
 };
 static_assert(sizeof(ArcItem) == 32, "arc item is 32 bytes");
 
+// Values of one launch at most: an event's id holds value << 3 | form in 28 bits.
+constexpr uint64_t kArcValuesMost = 1ull << 25;
+
 struct ArcConfig {
     int threads;      // CTA size (512 or 768)
     int ctas;         // persistent grid size

@@ -138,7 +138,7 @@ void ArcPlanner::take(const ArcPlanner& from, size_t i0, size_t i1) {
 bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target) {
     items.clear();
     groups_.clear();
-    if (rows.over() || keys_.over() || rest.over()) return false;
+    if (rows.over() || keys_.over() || rest.over() || entries > kArcValuesMost) return false;
     if (rows.empty()) return true;
     sort();
     if (order_.over() || sorted_.over()) return false;

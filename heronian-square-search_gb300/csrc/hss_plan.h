@@ -83,7 +83,8 @@ class ArcPlanner {
     void add(const RowInfo& R, uint32_t row, uint64_t limit, uint32_t max_exponent, uint64_t m0, uint64_t m1,
              uint64_t least);
     // Orders the rows, assigns their values' entries and builds the items.
-    // False when an array over given memory had no room.
+    // False when an array over given memory had no room, or for more values than
+    // kArcValuesMost.
     bool finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target);
     // Orders the rows as finish does, and takes rows [i0, i1) of another planner.
     void sort();

@@ -1,0 +1,104 @@
+// The planner of the arc path on the host: rows and items over a block plan cut
+// here, in equal pieces, from the segment offsets.
+#include "../../heronian-square-search_gb300/csrc/hss_plan.h"
+
+#include <cstdio>
+#include <cstdlib>
+
+#include "../../heronian-square-search_gb300/csrc/hss_prep.h"
+
+using namespace hss;
+
+#define CHECK(cond, ...)                                            \
+    do {                                                            \
+        if (!(cond)) {                                              \
+            std::printf("%s:%d: %s: ", __FILE__, __LINE__, #cond);  \
+            std::printf(__VA_ARGS__);                               \
+            std::printf("\n");                                      \
+            std::exit(1);                                           \
+        }                                                           \
+    } while (0)
+
+namespace {
+
+constexpr uint64_t kLimit = 100000;
+constexpr uint32_t kCtas = 152;
+HostCache cache;
+
+ArcPlan make_plan() {
+    const TypeTables types = make_type_tables();
+    ArcPlan plan;
+    for (uint32_t t = 0; t < kTypes; ++t) {
+        plan.type_first[t] = (uint32_t)plan.blocks.size();
+        const uint32_t roots = roots_upto(types, t, (uint32_t)kLimit);
+        for (uint32_t r0 = 0; r0 < roots; r0 += 400) {
+            const uint32_t r1 = std::min(roots, r0 + 400);
+            ArcBlock b{};
+            b.type = t;
+            b.rank0 = r0;
+            b.n_m = r1 - r0;
+            b.m_lo = nth_root(types, t, r0);
+            b.m_hi = nth_root(types, t, r1 - 1);
+            for (uint32_t r = r0; r < r1; ++r) {
+                const uint32_t m = nth_root(types, t, r);
+                b.n += cache.seg_off[m + 1] - cache.seg_off[m];
+            }
+            plan.blocks.push_back(b);
+        }
+    }
+    plan.type_first[kTypes] = (uint32_t)plan.blocks.size();
+    while ((kLimit >> plan.start_shift) > 4096) ++plan.start_shift;
+    for (uint32_t t = 0; t < kTypes; ++t) {
+        uint32_t b = plan.type_first[t];
+        for (uint64_t i = 0; i <= kLimit >> plan.start_shift; ++i) {
+            while (b < plan.type_first[t + 1] && plan.blocks[b].m_hi < i << plan.start_shift) ++b;
+            plan.start[t].push_back(b);
+        }
+    }
+    return plan;
+}
+
+// The constants of a root that the planner reads.
+RowInfo row_info(uint64_t l) {
+    RowInfo R{};
+    R.l = l;
+    R.l2 = l * l;
+    R.l4 = (unsigned __int128)R.l2 * R.l2;
+    R.n4 = (unsigned __int128)(kLimit * kLimit) * (kLimit * kLimit);
+    R.l3 = l % 3 == 0;
+    R.l5 = l % 5 == 0;
+    R.free_l = cache.seg_off[l + 1] - cache.seg_off[l] - 1;
+    const NumberFactors f = factor_number(cache.spf.data(), l);
+    R.nsplit = f.count;
+    for (uint32_t i = 0; i < f.count; ++i) {
+        R.sp[i] = f.primes[i];
+        R.se[i] = f.exps[i];
+    }
+    return R;
+}
+
+void add(ArcPlanner& p, uint64_t first, uint64_t last) {
+    for (uint64_t l = first; l <= last; ++l)
+        p.add(row_info(l), (uint32_t)(l - first), kLimit, cache.max_exponent, 1, kLimit, min_roots(kLimit, last - first + 1));
+}
+
+// A term's id holds its value's number in 28 bits, beside three of its form.
+void check_value_ids(const ArcPlan& plan) {
+    ArcPlanner p;
+    add(p, 1000, 1010);
+    p.entries = (uint64_t)1 << 25;
+    CHECK(p.finish(plan, kCtas, 0), "2^25 values have ids");
+    p.entries += 1;
+    CHECK(!p.finish(plan, kCtas, 0), "one more has none");
+}
+
+}  // namespace
+
+int main() {
+    std::string err;
+    CHECK(build_host_cache(kLimit, 8, &cache, &err) == 0, "host cache");
+    const ArcPlan plan = make_plan();
+    check_value_ids(plan);
+    std::printf("ok\n");
+    return 0;
+}

@@ -23,6 +23,6 @@ def run_native(tmp_path, name):
     assert ran.returncode == 0, ran.stdout + ran.stderr
 
 
-@pytest.mark.parametrize("name", ["growth", "pressure", "open"])
+@pytest.mark.parametrize("name", ["growth", "pressure", "open", "planner"])
 def test_host_side(tmp_path, name):
     run_native(tmp_path, name)
