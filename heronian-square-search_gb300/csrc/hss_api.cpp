@@ -549,9 +549,6 @@ int run_products(hss_t* h, const std::vector<RowRef>& rows) {
     return HSS_OK;
 }
 
-// An item's weight in evaluations as arc cost (a row value against a block: about 2^13 terms).
-uint64_t arc_item_target(const hss_opts& o) { return o.item_target >> 13; }
-
 // Launches the batched sequence for the rows collected in h->planner: reset
 // cursors and queues, rows and items H2D, the rows' values, the persistent
 // kernel, the shared-prime kernels over the rest list (when it holds any) and

@@ -17,6 +17,10 @@
 #include "hss_plan.h"
 
 namespace hss {
+// The item weight of a handle's options, in evaluations, as arc cost (a row value
+// against a block: about 2^13 terms); 0 leaves it to the planner.
+inline uint64_t arc_item_target(const hss_opts& o) { return o.item_target ? std::max(1u, o.item_target >> 13) : 0u; }
+
 struct Request;
 
 // First-fit allocator of row records in the serving state arena (host-side

@@ -302,7 +302,7 @@ int run_arc_group(hss_t* h, unsigned char* base, uint32_t rows, uint32_t lo, uin
         if (i0) NA_CUDA(cudaStreamSynchronize(st));
         for (; i1 > i0; i1 = i0 + (i1 - i0) / 2) {
             g_launch.take(g_plan, i0, i1);
-            if (g_launch.finish(*h->plan, (uint32_t)cfg.ctas, h->opts.item_target >> 13)) break;
+            if (g_launch.finish(*h->plan, (uint32_t)cfg.ctas, arc_item_target(h->opts))) break;
         }
         if (i1 == i0) {
             NA_CUDA(cudaStreamSynchronize(st));

@@ -192,8 +192,11 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
     // at LIMIT 10^6 (15.1 ms, now 11.6), 81 % of 16,384 rows' at 10^5 (154 ms, 132), 83 % of a
     // heavy root's at 10^7 (25 ms, 23).
     const uint64_t share12 = total / ((uint64_t)ctas * 12), share64 = total / ((uint64_t)ctas * 64);
-    const uint64_t target =
-        std::max<uint64_t>(16, item_target ? item_target : std::max(share64, std::min<uint64_t>(share12, kSmallItem)));
+    // A caller's size is not followed below a 2^17th of the launch's work: each
+    // item is 32 bytes of host and device memory (3,000 rows at LIMIT 10^5 would make
+    // 480,000 of cost 16), and callers without the power to allocate have room for 2^18.
+    const uint64_t target = std::max<uint64_t>(
+        16, item_target ? std::max(item_target, total >> 17) : std::max(share64, std::min<uint64_t>(share12, kSmallItem)));
     const uint64_t merged = std::min(std::max(target, std::min<uint64_t>(total / ctas, 400)), kMergedCost);
     Store<ArcItem>& cut = cut_;
     Store<uint32_t>& cut_lo = cut_lo_;

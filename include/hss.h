@@ -56,7 +56,8 @@ typedef struct {
                                  short calls), 512 picks 16 warps per CTA and
                                  anything else 24 */
     uint32_t item_target;     /* batched item weight in alpha*beta evaluations
-                                 (0: 1<<23; by arcs, chosen from the call's work) */
+                                 (0: 1<<23; by arcs, chosen from the call's work,
+                                 and not followed below a 2^17th of it) */
     uint32_t ctas_per_sm;     /* product kernel variant: minimum CTAs per SM it is
                                  compiled for (128 threads: 4 or 6; 256: 2 or 3;
                                  512: 1); 0 picks 4 / 2 / 1 */

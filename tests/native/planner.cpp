@@ -92,6 +92,23 @@ void check_value_ids(const ArcPlan& plan) {
     CHECK(!p.finish(plan, kCtas, 0), "one more has none");
 }
 
+// However small an item the caller asks for, their number stays within what
+// a launch's host and device memory hold.
+void check_item_weight(const ArcPlan& plan) {
+    ArcPlanner coarse, fine, fit;
+    add(coarse, 10000, 12999);
+    add(fine, 10000, 12999);
+    CHECK(coarse.finish(plan, kCtas, (uint64_t)1 << 40) && fine.finish(plan, kCtas, 1), "two weights");
+    CHECK(fine.items.size() > coarse.items.size(), "%zu and %zu items", fine.items.size(), coarse.items.size());
+    CHECK(fine.items.size() <= coarse.items.size() + ((size_t)1 << 18), "%zu items, %zu at least", fine.items.size(),
+          coarse.items.size());
+    // a caller without the power to allocate has room for 2^18: a heavy root fits
+    static ArcPlanner::Arena<8192, 1 << 18> arena;
+    fit.use(arena);
+    add(fit, 32045, 32045);
+    CHECK(fit.finish(plan, kCtas, 1), "a heavy root's items");
+}
+
 }  // namespace
 
 int main() {
@@ -99,6 +116,7 @@ int main() {
     CHECK(build_host_cache(kLimit, 8, &cache, &err) == 0, "host cache");
     const ArcPlan plan = make_plan();
     check_value_ids(plan);
+    check_item_weight(plan);
     std::printf("ok\n");
     return 0;
 }

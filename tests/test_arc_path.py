@@ -29,6 +29,11 @@ FIELDS = ("pairs", "processed", "products", "candidates", "r16", "merged", "merg
     (100_003, 64_080, 64_110, {"use_graph": 1}),
     (300_017, 160_215, 160_235, {}),
     (1_000_000, 801_120, 801_125, {}),
+    # item weights from the finest cut (2^17 items a launch) to one item per block; heavy rows over several items
+    (100_003, 32_032, 32_052, {"item_target": 1}),
+    (100_003, 32_032, 32_152, {"item_target": 1 << 31}),
+    (300_017, 160_215, 160_235, {"item_target": 1 << 17, "block_threads": 512}),
+    (1_000_000, 801_125, 801_125, {"item_target": 1 << 20, "block_threads": 512}),
 ])
 def test_batched_equals_plain(limit, first, last, opts):
     with hss.Search(limit, **opts) as s:
