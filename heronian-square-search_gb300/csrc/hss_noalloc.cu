@@ -281,7 +281,7 @@ int run_arc_group(hss_t* h, unsigned char* base, uint32_t rows, uint32_t lo, uin
         g_plan.add(g_host_rows[pc.r], pc.r, h->limit, h->dev.max_exponent, pc.m0, pc.m1 - 1, 1);
     }
     if (g_plan.rows.over() || g_plan.rest_pairs) return kNoRoom;
-    g_plan.sort();
+    if (!g_plan.sort()) return kNoRoom;
     ArcBuffers b{scratch_buffers(h, base), reinterpret_cast<const ArcRow*>(base + kOffArcRows),
                  reinterpret_cast<ArcValue*>(base + kOffArcValues), reinterpret_cast<HotRec*>(base + kOffArcHot),
                  h->d_arc_tabs};

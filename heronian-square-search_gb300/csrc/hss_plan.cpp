@@ -112,10 +112,13 @@ void ArcPlanner::add(const RowInfo& R, uint32_t row, uint64_t limit, uint32_t ma
 }
 
 // Rows by (P, parity, divisibility by 3 and 5), those of many values first.
-void ArcPlanner::sort() {
+bool ArcPlanner::sort() {
     const size_t n = rows.size();
+    order_.clear();
+    sorted_.clear();
     order_.resize(n);
     sorted_.resize(n);
+    if (order_.over() || sorted_.over() || keys_.over()) return false;
     for (size_t i = 0; i < n; ++i) order_[i] = Order{keys_[i], (uint64_t)(UINT32_MAX - rows[i].na) << 32 | i};
     std::sort(order_.begin(), order_.end(),
               [](const Order& x, const Order& y) { return x.key != y.key ? x.key < y.key : x.rest < y.rest; });
@@ -124,6 +127,7 @@ void ArcPlanner::sort() {
         keys_[i] = order_[i].key;
     }
     rows.swap(sorted_);
+    return true;
 }
 
 void ArcPlanner::take(const ArcPlanner& from, size_t i0, size_t i1) {
@@ -140,8 +144,7 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
     groups_.clear();
     if (rows.over() || keys_.over() || rest.over() || entries > kArcValuesMost) return false;
     if (rows.empty()) return true;
-    sort();
-    if (order_.over() || sorted_.over()) return false;
+    if (!sort()) return false;
     uint32_t ent = 0;
     for (size_t i = 0; i < rows.size(); ++i) {
         rows[i].ent = ent;
@@ -186,6 +189,7 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
         groups_.push_back(g);
         g0 = g1;
     }
+    if (groups_.over()) return false;
     // Item size: the caller's, or a sixty-fourth of a CTA's work, but not below
     // kSmallItem unless that leaves a CTA fewer than twelve items.  With twelve items
     // in every call the last ones ran alone, and CTAs worked 77 % of the time of 64 rows

@@ -3,6 +3,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <exception>
 #include <vector>
 
 #include "hss_blocks.h"
@@ -11,7 +12,8 @@
 namespace hss {
 
 // The planner's arrays: grown as needed, or over memory that is given once and
-// never exceeded (over() then tells that an entry found no room).
+// never exceeded.  over() tells that an entry found no room (in the given memory, or
+// in the host's: no exception leaves the planner, which C callers reach).
 template <class T>
 class Store {
   public:
@@ -56,7 +58,12 @@ class Store {
             over_ = true;
             return false;
         }
-        own_.resize(std::max(n, 2 * cap_));
+        try {
+            own_.resize(std::max(n, 2 * cap_));
+        } catch (const std::exception&) {  // bad_alloc, length_error
+            over_ = true;
+            return false;
+        }
         p_ = own_.data();
         cap_ = own_.size();
         return true;
@@ -83,11 +90,11 @@ class ArcPlanner {
     void add(const RowInfo& R, uint32_t row, uint64_t limit, uint32_t max_exponent, uint64_t m0, uint64_t m1,
              uint64_t least);
     // Orders the rows, assigns their values' entries and builds the items.
-    // False when an array over given memory had no room, or for more values than
-    // kArcValuesMost.
+    // False when an array had no room, or for more values than kArcValuesMost.
     bool finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target);
-    // Orders the rows as finish does, and takes rows [i0, i1) of another planner.
-    void sort();
+    // Orders the rows as finish does (false without room for it), and takes rows
+    // [i0, i1) of another planner.
+    bool sort();
     void take(const ArcPlanner& from, size_t i0, size_t i1);
 
     // Arrays over given memory, for callers that may not allocate.

@@ -4,6 +4,7 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <new>
 
 #include "../../heronian-square-search_gb300/csrc/hss_prep.h"
 
@@ -18,6 +19,17 @@ using namespace hss;
             std::exit(1);                                           \
         }                                                           \
     } while (0)
+
+namespace {
+size_t g_largest = ~size_t(0);  // allocations beyond this are refused
+}
+void* operator new(size_t n) {
+    void* p = n > g_largest ? nullptr : std::malloc(n);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 namespace {
 
@@ -109,6 +121,30 @@ void check_item_weight(const ArcPlan& plan) {
     CHECK(fit.finish(plan, kCtas, 1), "a heavy root's items");
 }
 
+// Host memory that runs out, at any size of the planner's arrays, is an answer
+// and no exception; the planner works again with memory.
+void check_memory(const ArcPlan& plan) {
+    ArcPlanner p;
+    for (size_t most = 64; most < (1u << 24); most *= 2) {
+        bool planned = false;
+        g_largest = most;
+        try {
+            p = ArcPlanner();
+            p.clear();
+            add(p, 10000, 10999);
+            planned = p.finish(plan, kCtas, 0);
+        } catch (const std::bad_alloc&) {
+            g_largest = ~size_t(0);
+            CHECK(false, "an exception with arrays of at most %zu bytes", most);
+        }
+        g_largest = ~size_t(0);
+        CHECK(!planned || most > 64, "planned in %zu bytes", most);
+    }
+    p.clear();
+    add(p, 10000, 10999);
+    CHECK(p.finish(plan, kCtas, 0), "with memory");
+}
+
 }  // namespace
 
 int main() {
@@ -117,6 +153,7 @@ int main() {
     const ArcPlan plan = make_plan();
     check_value_ids(plan);
     check_item_weight(plan);
+    check_memory(plan);
     std::printf("ok\n");
     return 0;
 }
