@@ -412,7 +412,9 @@ int build_arc_layout(const DeviceCache& cache, uint64_t records, const ArcPlan& 
                             cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess && !plan.blocks.empty()) {
         const size_t smem = block_sort_smem(plan.cap);
-        e = cudaFuncSetAttribute((const void*)block_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // (the limit is the kernel's, for every thread of the process: the same at every launch)
+        e = cudaFuncSetAttribute((const void*)block_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)block_sort_smem(kBlockEntries));
         if (e == cudaSuccess) {
             block_sort_kernel<<<(unsigned)plan.blocks.size(), kBlockThreads, smem, stream>>>(
                 out->blocks, plan.cap, cache.seg_off, cache.hot, cache.exact, cache.owner, out->w[0], out->w[1], out->w[2],

@@ -2240,9 +2240,20 @@ static const void* batched_fn(int threads, int min_blocks) {
     return min_blocks >= 3 ? (const void*)batched_kernel<256, 3> : (const void*)batched_kernel<256, 2>;
 }
 
+// Lets a kernel whose dynamic shared memory depends on its rows have all there
+// is.  The limit is the kernel's, for every thread of the process: with the
+// launch's own size, another thread's smaller one could come between.
+static cudaError_t allow_dynamic_smem(const void* fn) {
+    constexpr int kOptIn = 227 * 1024;
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, fn);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kOptIn - (int)a.sharedSizeBytes);
+}
+
 int batched_max_ctas_per_sm(int threads, int min_blocks, size_t smem) {
     const void* fn = batched_fn(threads, min_blocks);
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_dynamic_smem(fn);
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
@@ -2252,7 +2263,7 @@ cudaError_t launch_batched(const DeviceCache& cache, const WorkItem* items, uint
                            const BatchedConfig& cfg, const LaunchBuffers& buf, cudaStream_t stream) {
     size_t smem = batched_smem_bytes(cfg.threads, cfg.alpha_cap);
     const void* fn = batched_fn(cfg.threads, cfg.min_blocks);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(fn);
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&cache, (void*)&items, (void*)&n_items, (void*)&cfg.alpha_cap, (void*)&buf};
     return cudaLaunchKernel(fn, dim3(cfg.ctas), dim3(cfg.threads), args, smem, stream);
@@ -2262,8 +2273,7 @@ cudaError_t launch_plain(const DeviceCache& cache, uint64_t first_l, uint32_t n_
                          const LaunchBuffers& buf, cudaStream_t stream) {
     (void)first_l;
     size_t smem = (size_t)alpha_cap * sizeof(AlphaHot) + kTableBytes;
-    cudaError_t e = cudaFuncSetAttribute((const void*)plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_dynamic_smem((const void*)plain_kernel);
     if (e != cudaSuccess) return e;
     plain_kernel<<<n_rows * kSlices, kPlainThreads, smem, stream>>>(cache, alpha_cap, buf);
     return cudaGetLastError();
