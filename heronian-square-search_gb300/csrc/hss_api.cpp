@@ -632,8 +632,10 @@ constexpr size_t kLongCall = 2048;
 // time on launches and waits, of which the arc path has fewer (four roots at
 // 8000: 0.36 ms by products, 0.13 by arcs; one at 2000 or 5000: 0.29 and 0.25, 0.39 and
 // 0.18).
+bool goes_by_arcs(const hss_t* h, size_t rows) { return h->plan && (h->limit >= kArcLimit || rows <= kArcRows); }
+
 int run_batched(hss_t* h, const std::vector<RowRef>& rows) {
-    if (!h->plan || (h->limit < kArcLimit && rows.size() > kArcRows)) return run_products(h, rows);
+    if (!goes_by_arcs(h, rows.size())) return run_products(h, rows);
     h->planner.clear();
     size_t start = 0;
     bool grown = false;
@@ -1162,32 +1164,58 @@ extern "C" {
 int hss_autotune(hss_t* h, uint64_t first, uint64_t last, hss_opts* best, hss_tune_trial* trials,
                  uint32_t max_trials, uint32_t* ntrials) {
     if (!h) return HSS_ERR_ARGUMENT;
-    static const uint32_t kVariants[][2] = {{128, 4}, {128, 6}, {256, 2}, {256, 3}, {512, 1}};
-    static const uint32_t kTargets[] = {1u << 21, 1u << 22, 1u << 23, 1u << 24, 1u << 25};
+    struct Setting {
+        uint32_t threads, ctas, target;
+    };
+    static const uint32_t kProducts[][2] = {{128, 4}, {128, 6}, {256, 2}, {256, 3}, {512, 1}};
+    static const uint32_t kArcs[][2] = {{256, 2}, {512, 1}};  // 24 warps per CTA, and 16
+    static const uint32_t kTargets[] = {0, 1u << 21, 1u << 22, 1u << 23, 1u << 24, 1u << 25};
     const hss_opts saved = h->opts;
+    const bool arcs = first <= last && goes_by_arcs(h, last - first + 1);
+    // the handle's own setting first, then every variant with every weight; the
+    // product path's own weight is one of the list, the arc path's is 0
+    Setting list[1 + 5 * 6];
+    uint32_t n = 0;
+    auto add = [&](const Setting& x) {
+        for (uint32_t i = 0; i < n; ++i)
+            if (list[i].threads == x.threads && list[i].ctas == x.ctas && list[i].target == x.target) return;
+        list[n++] = x;
+    };
+    {
+        const uint32_t threads = arcs ? (saved.block_threads == 512 ? 512u : 256u) : saved.block_threads ? saved.block_threads : 256u;
+        const uint32_t ctas = !arcs && saved.ctas_per_sm ? saved.ctas_per_sm : threads == 128 ? 4u : threads == 512 ? 1u : 2u;
+        add(Setting{threads, ctas, saved.item_target || arcs ? saved.item_target : kDefaultItemTarget});
+    }
+    for (uint32_t v = 0; v < (arcs ? 2u : 5u); ++v) {
+        const uint32_t* variant = arcs ? kArcs[v] : kProducts[v];
+        for (uint32_t target : kTargets)
+            if (target || arcs) add(Setting{variant[0], variant[1], target});
+    }
     hss_opts chosen = saved;
     float best_ms = 0;
-    uint32_t n = 0;
-    for (const auto& v : kVariants)
-        for (uint32_t target : kTargets) {
-            h->opts.block_threads = v[0];
-            h->opts.ctas_per_sm = v[1];
-            h->opts.item_target = target;
-            hss_counts c;
-            int s = hss_search(h, first, last, HSS_MODE_BATCHED, &c, nullptr, nullptr, 0, nullptr);  // warm
-            if (!s) s = hss_search(h, first, last, HSS_MODE_BATCHED, &c, nullptr, nullptr, 0, nullptr);
-            if (s) {
-                h->opts = saved;
-                return s;
-            }
-            float ms = (float)c.kernel_ms;
-            if (trials && n < max_trials) trials[n] = hss_tune_trial{v[0], v[1], target, ms};
-            ++n;
-            if (best_ms == 0 || ms < best_ms) {
-                best_ms = ms;
-                chosen = h->opts;
-            }
+    for (uint32_t i = 0; i < n; ++i) {
+        h->opts.block_threads = list[i].threads;
+        h->opts.ctas_per_sm = list[i].ctas;
+        h->opts.item_target = list[i].target;
+        hss_counts c;
+        int s = hss_search(h, first, last, HSS_MODE_BATCHED, &c, nullptr, nullptr, 0, nullptr);  // warm
+        if (!s) s = hss_search(h, first, last, HSS_MODE_BATCHED, &c, nullptr, nullptr, 0, nullptr);
+        if (s) {
+            h->opts = saved;
+            return s;
         }
+        float ms = (float)c.kernel_ms;
+        if (trials && i < max_trials) trials[i] = hss_tune_trial{list[i].threads, list[i].ctas, list[i].target, ms};
+        // By arcs a weight holds for calls of every size from then on, where the
+        // planner's follows the call: it has to be worth 3 % (runs of one setting
+        // differ by 2 %; at LIMIT 10^7 64 roots take 16.4 ms by the planner's and 16.4
+        // to 17.8 ms with fixed ones, 512 roots 106.1 to 108.5 ms and 106.1 to 122.3).
+        if (arcs && list[i].target) ms *= 1.03f;
+        if (best_ms == 0 || ms < best_ms) {
+            best_ms = ms;
+            chosen = h->opts;
+        }
+    }
     h->opts = chosen;
     if (best) *best = chosen;
     if (ntrials) *ntrials = n;

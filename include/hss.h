@@ -179,9 +179,13 @@ int hss_search(hss_t* h, uint64_t first, uint64_t last, int mode, hss_counts* ou
                uint64_t* row_candidates, hss_hit* hits, uint32_t hit_cap, uint32_t* nhits);
 
 /* Autotuner: times the batched path on rows first..last (a sample of the
- * intended workload) for every compiled kernel variant (CTA size and minimum
- * CTAs per SM, which caps registers per thread) and item weight, keeps the
- * fastest configuration in the handle's options and returns it in *best.
+ * intended workload) with the handle's own options, then for every compiled
+ * kernel variant of the sample's path (products: CTA size and minimum CTAs per SM,
+ * which caps registers per thread; arcs: 24 or 16 warps per CTA, reported as 256
+ * and 512 threads) and item weight, keeps the fastest configuration in the
+ * handle's options and returns it in *best.  By arcs an item target of 0, the
+ * choice from each call's work, is among them, and a fixed one is taken when it is
+ * more than 3 % faster on the sample.
  * `trials` receives up to max_trials (threads, ctas_per_sm, item_target,
  * milliseconds) records when not NULL. */
 typedef struct {

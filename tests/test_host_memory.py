@@ -23,7 +23,7 @@ def run_native(tmp_path, name, parts):
     assert ran.returncode == 0, ran.stdout + ran.stderr
 
 
-@pytest.mark.parametrize("name", ["growth", "pressure", "open", "planner"])
+@pytest.mark.parametrize("name", ["growth", "pressure", "open", "planner", "autotune"])
 def test_host_side(tmp_path, name):
     run_native(tmp_path, name, [CSRC / "hss_plan.cpp", CSRC / "hss_prep.cpp"])
 
