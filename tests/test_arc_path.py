@@ -29,6 +29,12 @@ FIELDS = ("pairs", "processed", "products", "candidates", "r16", "merged", "merg
     (100_003, 64_080, 64_110, {"use_graph": 1}),
     (300_017, 160_215, 160_235, {}),
     (1_000_000, 801_120, 801_125, {}),
+    # calls with a hit (1853, 4380, 4427), (11789, 68104, 68595)
+    (5_000, 1_850, 1_860, {}),
+    (70_000, 11_789, 11_789, {}),
+    (70_000, 11_750, 11_850, {"use_graph": 1}),
+    # the largest limit: low roots with the longest shared-prime rows
+    (30_000_000, 1_104, 1_105, {}),
     # item weights from the finest cut (2^17 items a launch) to one item per block; heavy rows over several items
     (100_003, 32_032, 32_052, {"item_target": 1}),
     (100_003, 32_032, 32_152, {"item_target": 1 << 31}),
@@ -95,3 +101,31 @@ def test_queues_grow_from_their_first_size(plain_long, form):
     assert larger <= grown / 2 ** 20 < larger + 1024
     assert {k: counts[k] for k in FIELDS} == {k: plain_long.counts[k] for k in FIELDS}
     assert sorted(hits) == sorted(plain_long.hits)
+
+
+@pytest.mark.gpu
+def test_rest_list_equals_rows_at_the_largest_limit():
+    """A call of 65 roots leaves the common parts with few roots to the shared-prime kernels; calls of 64 and of one root
+    make rows of all of them."""
+    with hss.Search(30_000_000) as s:
+        whole = s.search(1_041, 1_105, rows=True)
+        parts = [s.search(1_041, 1_104, rows=True), s.search(1_105, 1_105, rows=True)]
+    for key in FIELDS:
+        assert whole.counts[key] == sum(p.counts[key] for p in parts), key
+    assert whole.row_candidates == parts[0].row_candidates + parts[1].row_candidates
+    assert whole.counts["launches"] > parts[0].counts["launches"]
+
+
+@pytest.mark.gpu
+def test_root_of_the_most_values(built):
+    """15,413,645 has the most values of all roots with its common parts (13.3 M at the largest limit; with itself it shares
+    all five split primes).  Its pairs up to 15,420,000 against the oracle."""
+    from oracle import Oracle
+    limit, root = 15_420_000, 15_413_645
+    with Oracle(limit) as o:
+        want = o.search(root, root)
+    with hss.Search(limit) as s:
+        got = s.search(root, root, rows=True)
+    for key in ("pairs", "processed", "products", "candidates", "r16"):
+        assert got.counts[key] == want[key], key
+    assert got.row_candidates == want["row_candidates"]
