@@ -808,7 +808,6 @@ int open_arc_layout(hss_t* h) {
     h->dev.arc_index = b.index;
     h->dev.arc_mask = b.mask;
     h->dev.pos = b.pos;
-    h->dev.block_cap = plan->cap;
     h->plan = std::move(plan);
     return HSS_OK;
 }

@@ -119,18 +119,13 @@ static_assert(sizeof(DevHit) == 48, "hit record is 48 bytes");
 // 2^10, each the product of two primes, so that a value's (re, im) and its
 // root's m^4 fit one 32-bit word per field.
 constexpr uint32_t kFields = 3;
-constexpr uint32_t kFieldMod[kFields] = {17 * 37, 13 * 61, 11 * 73};
 HSS_HD constexpr uint32_t field_mod(uint32_t f) { return f == 0 ? 17 * 37 : f == 1 ? 13 * 61 : 11 * 73; }
 // ceil(2^32 / M): multiplying by it maps t mod M to the top bits of a word
 HSS_HD constexpr uint32_t field_scale(uint32_t f) { return 0xFFFFFFFFu / field_mod(f) + 1u; }
 
 // Roots m by divisibility: 3 classes by powers of two (odd, 2 mod 4, 0 mod 4)
-// times divisibility by 3 and by 5.
+// times divisibility by 3 and by 5, numbered 4 class + 2 (3 divides m) + (5 divides m).
 constexpr uint32_t kTypes = 12;
-HSS_HD inline uint32_t type_of(uint32_t m) {
-    const uint32_t v = (m & 1u) ? 0u : (m & 3u) ? 1u : 2u;
-    return v * 4u + (m % 3u == 0 ? 2u : 0u) + (m % 5u == 0 ? 1u : 0u);
-}
 
 // The roots of a type repeat with period 60: their residues in 1..60 order,
 // and how many of them are at most r, for r = 0..59.
@@ -226,7 +221,6 @@ struct ArcCache : DeviceCache {
     const float2* arc_xy;       // its value (positive imaginary part)
     const uint32_t* arc_mask;   // kMaskPrimes * kMaskWords per block
     const uint16_t* pos;
-    uint32_t block_cap;         // entries of the largest block
 };
 
 // Offset of exponent e's 4e+1 values within prime p's block:
