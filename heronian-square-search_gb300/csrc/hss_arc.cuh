@@ -31,13 +31,15 @@
 //
 // What bounds it: instruction issue (64 rows at LIMIT 10^6: 68 % of the issue
 // slots while an SM is busy, 27 of 32 lanes; DRAM under 1 %: a block is read
-// once per item, 53 bytes an entry, for a million tests and more).  One CTA of
+// once per item, 17 bytes an entry, for a million tests and more).  One CTA of
 // 24 warps per SM, since the block of 6144 entries and the warps' own staging
 // fill its shared memory; two CTAs of 8 or 12 warps with smaller blocks were
 // slower (more runs per row).  Warps work on rows by themselves, with no barrier
 // but at a change of block.  In place of one test of every product (512 rows at
-// LIMIT 10^7, l = 7.5 10^6: 778 ms) the batch takes 106 ms; one root of branch
-// weight 625 takes 23 ms (87), 37 roots near the limit 1.35 ms (14.7).
+// LIMIT 10^7, l = 7.5 10^6: 778 ms) the batch takes 106 ms; root 6,325,815 (branch
+// weight 625) takes 22 ms (87), 37 roots near the limit 1.35 ms (14.7).
+// Of the batch's 86 G warp instructions some 29 G are the filter (1.03 G tests of 32
+// terms) and 9 G the starts of its 0.19 G runs.
 
 __constant__ TypeTables c_arc_types = make_type_tables();
 
@@ -282,7 +284,8 @@ __device__ __forceinline__ bool arc_prepare(const ArcCache& cache, const ArcBuff
     }
     // Small primes have their bit sets ready, so that most rows gather little or
     // nothing: three rows at LIMIT 10^7 (l = 160,000) 8.1 ms without them and 5.1 ms
-    // with, 37 near the limit 1.5 and 1.35, 512 rows 125 and 121.
+    // with, 37 near the limit 1.5 and 1.35; 512 rows, before their items were cut as
+    // now, 125 and 121.
     uint32_t small = __ballot_sync(kFull, multiples != 0 && p <= mask_prime(kMaskPrimes - 1));
     const bool masks = small != 0;
     uint32_t pick = 0, picked = 0;  // which of them, four bits each

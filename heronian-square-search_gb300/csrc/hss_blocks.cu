@@ -49,7 +49,7 @@ __device__ __forceinline__ uint32_t residue_i64(int64_t v, uint32_t m) {
 // every term between the tightest and the widest window of the block's roots (as
 // the square of the size over the root and the type's share of all roots), so the
 // best size grows as the square root of root times share (a factor of 3: 16,384
-// rows at LIMIT 10^5 132 ms, a heavy root at 10^7 23.2; of 2: 147 and 22.5, of 4.5:
+// rows at LIMIT 10^5 132 ms, root 6,325,815 at 10^7 23.2; of 2: 147 and 22.5, of 4.5:
 // 129 and 23.7).  Without `blocks` the warp's count is left in at[task], with
 // them they are written from there on.  0.2 ms each time at N = 10^7, where host
 // threads took 14 ms.

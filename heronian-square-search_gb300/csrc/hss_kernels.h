@@ -196,7 +196,8 @@ cudaError_t launch_batched(const DeviceCache& cache, const WorkItem* items, uint
                            const BatchedConfig& cfg, const LaunchBuffers& buf, cudaStream_t stream);
 
 // Plain kernel: rows first_l .. first_l + n_rows - 1, one block per
-// (row, slice) and one thread per pair (the reference's launch shape).
+// (row, slice), a lane per record of 32 pairs at a time (the reference's launch
+// shape has a thread per pair).
 cudaError_t launch_plain(const DeviceCache& cache, uint64_t first_l, uint32_t n_rows,
                          uint32_t alpha_cap, const LaunchBuffers& buf, cudaStream_t stream);
 

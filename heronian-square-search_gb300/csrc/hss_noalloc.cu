@@ -7,7 +7,8 @@
 // a pool or an embedding runtime fixed at start-up, or loops that cannot take
 // the implicit synchronisation an allocation brings.  hss_search_noalloc runs
 // the same batched launch sequence (by arcs where the handle has their layout: 8
-// rows at LIMIT 10^7 took 29.6 ms by products and take 5.0 ms; else the product,
+// rows of the reference batch at LIMIT 10^7 took 24.6 to 29.6 ms by products and
+// take 2.0 to 3.1 ms; else the product,
 // shared-prime and exact kernels) with all per-call device scratch in one file-scope array of
 // kNoAllocBytes that is part of the library image, and host staging in static
 // buffers.  Every GPU that loads the library holds the array until the process

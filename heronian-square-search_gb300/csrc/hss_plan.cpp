@@ -27,9 +27,9 @@ uint64_t fourth_root(u128 x) {
 // A row (l, P) costs its value list and a visit to every block of its range; the
 // shared-prime kernels set every pair up by itself, and cost three launches
 // that wait for one another.  Few rows: no shared-prime launch at all (37 roots at
-// LIMIT 10^7 1.8 ms against 2.2 ms with 48 roots, one at 70,000 0.21 against 0.28 ms).
-// Many: 48 (512 roots at 10^7 114.5 ms, against 117 ms with 1 and 114.4 with 150), at small
-// limits, whose blocks hold fewer roots each, 150 (2,001 roots at 20,000 6.1 ms against 6.9 ms with 48).
+// LIMIT 10^7 1.34 ms against 1.81 ms with 48 roots, one at 70,000 0.15 against 0.22 ms).
+// Many: 48 (512 roots at 10^7 106.1 ms, against 109.6 ms with 1 and 106.3 with 150), at small
+// limits, whose blocks hold fewer roots each, 150 (2,001 roots at 20,000 5.4 ms against 5.8 ms with 48).
 uint64_t min_roots(uint64_t limit, size_t rows) { return rows <= 64 ? 1 : limit < 1000000 ? 150 : 48; }
 
 void ArcPlanner::clear() {
@@ -193,8 +193,8 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
     // Item size: the caller's, or a sixty-fourth of a CTA's work, but not below
     // kSmallItem unless that leaves a CTA fewer than twelve items.  With twelve items
     // in every call the last ones ran alone, and CTAs worked 77 % of the time of 64 rows
-    // at LIMIT 10^6 (15.1 ms, now 11.6), 81 % of 16,384 rows' at 10^5 (154 ms, 132), 83 % of a
-    // heavy root's at 10^7 (25 ms, 23).
+    // at LIMIT 10^6 (15.1 ms, now 11.4), 81 % of 16,384 rows' at 10^5 (154 ms, 128), 83 % of
+    // root 6,325,815's (branch weight 625) at 10^7 (25 ms, 22).
     const uint64_t share12 = total / ((uint64_t)ctas * 12), share64 = total / ((uint64_t)ctas * 64);
     // A caller's size is not followed below a 2^17th of the launch's work: each
     // item is 32 bytes of host and device memory (3,000 rows at LIMIT 10^5 would make
@@ -213,9 +213,9 @@ bool ArcPlanner::finish(const ArcPlan& plan, uint32_t ctas, uint64_t item_target
     for (size_t x = 0; x < groups_.size();) {
         // Groups that fit one item together share it: a block is loaded and waited
         // for once for all of them.  With an item per group, three rows at LIMIT 10^7
-        // spent 43 to 79 % of their time on loads and barriers: 4.5 ms and 2.4 ms so
-        // (l = 331,000), 10.8 and 8.1 ms (l = 160,000); 8 rows at 7.5 10^6 4.8 and 2.9 ms,
-        // 37 near the limit 1.75 and 1.5 ms.  Groups above kMergedCost hold enough
+        // spent 43 to 79 % of their time on loads and barriers; when this came they went from
+        // 4.5 to 2.4 ms (l = 331,000) and 10.8 to 8.1 ms (l = 160,000), 8 rows at 7.5 10^6
+        // from 4.8 to 2.9 ms, 37 near the limit from 1.75 to 1.5 ms.  Groups above kMergedCost hold enough
         // work per block by themselves.
         size_t y = x + 1;
         uint64_t w = groups_[x].cost;

@@ -39,7 +39,7 @@ extern "C" {
 #define HSS_MAX_LIMIT 30000000ULL  /* every segment (<= 4063 values) fits a work item */
 
 /* Enumeration paths.  PLAIN mirrors the reference's launch shape (one block
- * per (root, slice), one thread per pair, gpu_search_v42.cu:298-304);
+ * per (root, slice), gpu_search_v42.cu:298-304; a lane per record of 32 pairs);
  * BATCHED is the persistent kernel draining a work queue of (root, m-range)
  * items weighted by Gaussian divisor count.  Both give identical counts. */
 #define HSS_MODE_PLAIN 0
